@@ -112,9 +112,9 @@ typedef struct {
                                  (where every row has at most 4,096 products and 1,280 A
                                  entries), 0 = per-segment pipeline */
     int32_t batch_warp_max;   /* threads per row in the persistent batch kernels: rows of at most
-                                 this many products (128..512, default 512) get one warp
-                                 (register sort), larger rows a 128-thread CTA (up to 1,024
-                                 products) or a 256-thread CTA (up to 4,096) */
+                                 this many products (128..512, default 512) get a warp (up to
+                                 256 products) or 64 threads, larger rows a 128-thread CTA (up
+                                 to 1,024 products) or a 512-thread CTA (up to 4,096) */
 } ops_tuning;
 int ops_handle_set_tuning(ops_handle_t handle, const ops_tuning *tuning);
 int ops_handle_get_tuning(ops_handle_t handle, ops_tuning *tuning);
@@ -130,13 +130,12 @@ int ops_handle_get_thresholds(ops_handle_t handle, int32_t *thresholds, int coun
 /* Message for the last failing call on this handle ("" if none). */
 const char *ops_handle_last_error(ops_handle_t handle);
 /* Rows handled by each sub-kernel in the last call (synchronises the handle's device
- * counters to the host): out[0..2] = E1 numeric rows by warp sort, warp hash and
- * expand/sort/compress; out[3..4] = E2 rows by the mid and the large expand/sort/compress
- * shape; out[5..6] = D rows by the whole-GPU sort and by the dense-row kernel;
- * out[7..9] = expand rows of the numeric phase whose columns span fewer than 65,536
- * columns, by path: column-window rank with no repeated column, rank with repeated
- * columns re-folded, sort (more than 128 products in repeated columns).  Diagnostic; no
- * OpSparse counterpart. */
+ * counters to the host): out[0..2] = E1 numeric rows by the small rank shapes (a warp or 64
+ * threads), warp hash and the 128-thread rank shape; out[3..4] = E2 rows by the mid and the
+ * large rank shape; out[5..6] = D rows by the whole-GPU sort and by the dense-row kernel;
+ * out[7..9] = rows of the 128-thread rank shape where B has at most 65,536 columns, by the
+ * products whose column another product of the row had before: none, 1 to 128, more.
+ * Diagnostic; no OpSparse counterpart. */
 int ops_handle_subclass_rows(ops_handle_t handle, int32_t *out, int count);
 const char *ops_status_string(int status);
 
@@ -244,8 +243,7 @@ int ops_batch_destroy(ops_batch_t batch);
 /* Chooses every field of ops_tuning for a workload by coordinate descent: the row-class
  * thresholds, the warp-hash table's slots per output entry (hash-table size), the batch
  * plan (persistent kernels over row-size queues, or per segment) and the largest row a warp
- * takes in the persistent kernels (threads per row: a warp, or a 128- or 256-thread CTA
- * above it).  Each candidate is timed as complete batched runs of `items` (a representative
+ * (or 64 threads) takes in the persistent kernels (a 128- or 512-thread CTA above it).  Each candidate is timed as complete batched runs of `items` (a representative
  * sample) with CUDA events, median of `reps` runs.  Installs the best tuning on the handle
  * (read it with ops_handle_get_tuning), returns its thresholds in best[6] and the time in
  * *best_ms.  Synchronizes.  No OpSparse counterpart: its tunables are compile-time

@@ -146,9 +146,10 @@ class Handle:
         return t.as_dict()
 
     def subclass_rows(self) -> dict:
-        """Rows per sub-kernel of the last call: E1 numeric (warp sort, warp hash,
-        expand/sort/compress), E2 (mid, large shape), D (whole-GPU sort, dense kernel), and
-        the expand rows of narrow column span by path (rank, rank with re-fold, sorted)."""
+        """Rows per sub-kernel of the last call: E1 numeric (small rank shapes, warp hash,
+        128-thread rank shape), E2 (mid, large shape), D (whole-GPU sort, dense kernel), and
+        the 128-thread shape's rows by repeated columns where B has at most 65,536 columns
+        (none, up to 128 products, more)."""
         arr = (C.c_int32 * 10)()
         check(self.lib.ops_handle_subclass_rows(self.h, arr, 10), self.h)
         return dict(zip(("e1_sort", "e1_hash", "e1_esc", "e2_mid", "e2_large", "d_sort", "d_dense", "rank",

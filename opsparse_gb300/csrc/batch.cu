@@ -212,7 +212,6 @@ struct ops_batch_s {
     // persistent path (batch_rows.cuh): one setup kernel, and one kernel per row-size queue
     // and phase, over every segment
     bool persistent = false;
-    bool key64 = false;            // numeric sort keys need 64 bits (a segment has > 2^20 columns)
     void *pmem = nullptr;          // queues, per-row products, segment arguments, scan scratch
     opsg::BatchQueues *q = nullptr;
     int *queues = nullptr;         // [kNumBatchQueues][total_rows] global row numbers
@@ -397,22 +396,23 @@ int launch_batch_symbolic(ops_batch_s *b, cudaStream_t st)
     return fork_queues(b, st, [&](int c, cudaStream_t s) {
         switch (c) {
             case kQ128:
-                return launch_queue(b, 0, c, k_batch_count_rows<2 * kBatchQ128>, kBatchCountThreads,
-                                    (size_t)W * 2 * kBatchQ128 * sizeof(int), a, s);
-            case kQWarp:  // twice the table a row needs: room for the wide column window
+                return launch_queue(b, 0, c, k_batch_rank_rows<RankW, false, double>, RankW::kThreads,
+                                    RankW::smem<false>(), a, s);
+            case kQ256:
+            case kQ512:  // twice the table a row needs: room for the wide column window
                 return launch_queue(b, 0, c, k_batch_count_rows<4 * kBatchWarpMax>, kBatchCountThreads,
                                     (size_t)W * 4 * kBatchWarpMax * sizeof(int), a, s);
             case kQE1:
-                return launch_queue(b, 0, c, k_batch_count_rows<2 * BescE1Batch::kCap>, kBatchCountThreads,
-                                    (size_t)W * 2 * BescE1Batch::kCap * sizeof(int), a, s);
-            default:  // the table and the A-entry scan of EscMid's symbolic shape
-                return launch_queue(b, 0, c, k_batch_cta_count, EscMid::kThreads,
-                                    (size_t)EscMid::kTable * 4 + (size_t)EscMid::kAEntries * 8, a, s);
+                return launch_queue(b, 0, c, k_batch_count_rows<2 * RankE1::kCap>, kBatchCountThreads,
+                                    (size_t)W * 2 * RankE1::kCap * sizeof(int), a, s);
+            default:
+                return launch_queue(b, 0, c, k_batch_rank_rows<RankMid, false, double>, RankMid::kThreads,
+                                    RankMid::smem<false>(), a, s);
         }
     });
 }
 
-template <typename T, typename KT>
+template <typename T>
 int launch_batch_numeric(ops_batch_s *b, cudaStream_t st)
 {
     static_assert(sizeof(SpgemmArgs<T>) == sizeof(SpgemmArgs<double>), "argument layout is the value type's");
@@ -420,17 +420,20 @@ int launch_batch_numeric(ops_batch_s *b, cudaStream_t st)
     return fork_queues(b, st, [&](int c, cudaStream_t s) {
         switch (c) {
             case kQ128:
-                return launch_queue(b, 1, c, k_batch_warp_rows<4, T, KT>, WsortShape<4>::kThreads,
-                                    WsortShape<4>::smem<true, T, KT>(), a, s);
-            case kQWarp:
-                return launch_queue(b, 1, c, k_batch_warp_rows<16, T, KT>, WsortShape<16>::kThreads,
-                                    WsortShape<16>::smem<true, T, KT>(), a, s);
+                return launch_queue(b, 1, c, k_batch_rank_rows<RankW, true, T>, RankW::kThreads, RankW::smem<true>(), a,
+                                    s);
+            case kQ256:
+                return launch_queue(b, 1, c, k_batch_rank_rows<RankS, true, T>, RankS::kThreads, RankS::smem<true>(), a,
+                                    s);
+            case kQ512:
+                return launch_queue(b, 1, c, k_batch_rank_rows<RankM, true, T>, RankM::kThreads, RankM::smem<true>(), a,
+                                    s);
             case kQE1:
-                return launch_queue(b, 1, c, k_batch_cta_rows<BescE1Batch, true, T, KT>, BescE1Batch::kThreads,
-                                    BescE1Batch::smem<true, KT, T>(), a, s);
+                return launch_queue(b, 1, c, k_batch_rank_rows<RankE1, true, T>, RankE1::kThreads,
+                                    RankE1::smem<true>(), a, s);
             default:
-                return launch_queue(b, 1, c, k_batch_cta_rows<BescMidRank, true, T, KT>, BescMidRank::kThreads,
-                                    BescMidRank::smem<true, KT, T>(), a, s);
+                return launch_queue(b, 1, c, k_batch_rank_rows<RankMid, true, T>, RankMid::kThreads,
+                                    RankMid::smem<true>(), a, s);
         }
     });
 }
@@ -446,11 +449,10 @@ int plan_persistent(ops_batch_s *b, ops_handle_s *h, size_t vs, cudaStream_t st,
     const int nseg = (int)b->segs.size();
     if (!h->batch_persistent || nseg == 0 || nseg > kBatchMaxSegs) return OPS_OK;
     long long total_rows = 0;
-    int max_m = 0, max_n = 0;
+    int max_m = 0;
     for (const Segment &s : b->segs) {
         total_rows += s.M;
         max_m = std::max(max_m, s.M);
-        max_n = std::max(max_n, s.N);
     }
     if (total_rows == 0 || total_rows > INT_MAX) return OPS_OK;
     size_t cub_bytes = 0;
@@ -540,7 +542,6 @@ int plan_persistent(ops_batch_s *b, ops_handle_s *h, size_t vs, cudaStream_t st,
         num[i] = seg_args<double>(s);  // the value pointers are reinterpreted by the value type
     }
     OPS_CUDA(h, cudaMemcpyAsync(b->d_num, num.data(), sizeof(SpgemmArgs<double>) * nseg, cudaMemcpyHostToDevice, st));
-    b->key64 = max_n > (1 << (32 - BescMidRank::kIdBits));  // the widest product index of the numeric keys
     b->persistent = true;
     used = true;
     return OPS_OK;
@@ -755,10 +756,8 @@ int record_numeric(ops_batch_s *b, cudaStream_t st)
         OPS_CUDA(h, cudaMemsetAsync(b->q->cursor[1], 0, sizeof(b->q->cursor[1]), st));
         OPS_CUDA(h, cudaMemsetAsync(b->segs[0].info, 0, sizeof(DevInfo) * b->segs.size(), st));
         if (b->dtype == OPS_F64)
-            return b->key64 ? launch_batch_numeric<double, unsigned long long>(b, st)
-                            : launch_batch_numeric<double, unsigned>(b, st);
-        return b->key64 ? launch_batch_numeric<float, unsigned long long>(b, st)
-                        : launch_batch_numeric<float, unsigned>(b, st);
+            return launch_batch_numeric<double>(b, st);
+        return launch_batch_numeric<float>(b, st);
     }
     for (Segment &s : b->segs) {
         if (s.count == 0) continue;
@@ -867,7 +866,7 @@ extern "C" int ops_batch_queues(ops_batch_t b, int32_t *persistent, int64_t *war
 {
     if (!b || !persistent || !warp_rows || !cta_rows) return OPS_INVALID_ARGUMENT;
     *persistent = b->persistent ? 1 : 0;
-    *warp_rows = b->persistent ? (int64_t)b->queue_rows[kQ128] + b->queue_rows[kQWarp] : 0;
+    *warp_rows = b->persistent ? (int64_t)b->queue_rows[kQ128] + b->queue_rows[kQ256] + b->queue_rows[kQ512] : 0;
     *cta_rows = b->persistent ? (int64_t)b->queue_rows[kQE1] + b->queue_rows[kQMid] : 0;
     return OPS_OK;
 }

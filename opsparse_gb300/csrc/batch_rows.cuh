@@ -3,45 +3,40 @@
 // A batch's problems are laid out as block-diagonal segments (see batch.cu).  Instead of
 // classifying each segment on its own and launching each class's kernels per segment, one
 // setup kernel walks the rows of every segment of every problem and pushes each row into one
-// of four global queues by its product count:
+// of five global queues by its product count:
 //   kQ128:  at most 128 products;
-//   kQWarp: 129 .. warp_max (<= 512) products;
+//   kQ256:  129 .. min(256, warp_max) products;
+//   kQ512:  257 .. warp_max (<= 512) products;
 //   kQE1:   warp_max+1 .. 1,024 products (and at most 1,024 A entries);
 //   kQMid:  1,025 .. 4,096 products (and at most 1,280 A entries).
-// Rows beyond all four are only counted; a batch that has any runs the per-segment pipeline
+// Rows beyond all five are only counted; a batch that has any runs the per-segment pipeline
 // instead.  Each queue is then drained by ONE persistent kernel per phase that spans every
 // problem: its warps (or CTAs) take rows through the queue's atomic cursor until it is
-// empty, with the shape and occupancy of its row size:
-//   symbolic  kQ128, kQWarp, kQE1: a warp per row, distinct columns counted in a shared-memory
-//             hash table of 2 slots per product (256, 1,024, 2,048 slots);
-//             kQMid: a 256-thread CTA per row, hash table of 2 slots per product (esc.cuh);
-//   numeric   kQ128: a warp per row, register bitonic network of up to 128 keys, 8 warps per
-//             CTA (wsort.cuh); kQWarp: the same with networks of up to 512 keys, 4 warps per
-//             CTA; kQE1: a 128-thread CTA per row (besc.cuh, 1,024 keys); kQMid: a 256-thread
-//             CTA per row (4,096 keys).
-// The four kernels of a phase run concurrently on their own streams.  The numeric routines
-// are the single-product kernels' (the same bits); every output entry is folded in
-// ascending j.
+// empty, with the rank shape (rank.cuh) of its row size: a warp (two shapes), 64, 128 or 512
+// threads per row.  In the symbolic phase the three middle queues count rows of long B rows
+// over a window bitmap, a warp per row.
+// The five kernels of a phase run concurrently on their own streams.  The row routines are
+// the single-product kernels' (the same bits); every output entry is folded in ascending j.
 //
 // Replaces, for a batch, OpSparse's per-bin dispatch (src/opsparse/core_algo/spgemm/
 // spgemm_phases.cu:52-121, 148-206), which launches each bin's kernel on its own stream for
 // one matrix at a time.
 #pragma once
 
-#include "besc.cuh"
-#include "wsort.cuh"
+#include "lists.cuh"
 
 namespace opsg {
 
-constexpr int kBatchQ128 = 128;       // rows of the kQ128 queue, at most (WsortShape<4>::kMax)
-constexpr int kBatchWarpMax = 512;    // rows of the kQWarp queue, at most (WsortShape<16>::kMax)
+constexpr int kBatchQ128 = 128;       // products of the kQ128 queue's rows, at most
+constexpr int kBatchQ256 = 256;       // products of the kQ256 queue's rows, at most
+constexpr int kBatchWarpMax = 512;    // products of the kQ512 queue's rows, at most
 constexpr int kBatchChunk = 8;        // warp-queue rows a warp takes per cursor step
 constexpr int kBatchMaxSegs = 16;     // segments one persistent launch covers (their arguments sit in shared memory)
 constexpr int kBatchCountThreads = 256;
-static_assert(WsortShape<4>::kMax == kBatchQ128 && WsortShape<16>::kMax == kBatchWarpMax, "warp-queue capacities");
-static_assert(EscMid::kProducts >= BescMidRank::kCap && EscMid::kAEntries >= BescMidRank::kAEntries, "kQMid rows fit both shapes");
+static_assert(RankW::kCap >= kBatchQ128 && RankS::kCap >= kBatchQ256 && RankM::kCap >= kBatchWarpMax,
+              "queue capacities");
 
-enum BatchQueue : int { kQ128 = 0, kQWarp = 1, kQE1 = 2, kQMid = 3, kQBeyond = 4, kNumBatchQueues = 4 };
+enum BatchQueue : int { kQ128 = 0, kQ256 = 1, kQ512 = 2, kQE1 = 3, kQMid = 4, kQBeyond = 5, kNumBatchQueues = 5 };
 
 // Device-side state of a batch's queues.
 struct BatchQueues {
@@ -98,9 +93,9 @@ static __global__ void __launch_bounds__(256) k_batch_setup(const SpgemmArgs<dou
             const_cast<int *>(g.row_flop)[r] = flop > INT_MAX ? INT_MAX : (int)flop;
             if (flop == 0) g.c_rpt[r] = 0;
             else if (flop <= kBatchQ128) cls = kQ128;
-            else if (flop <= warp_max) cls = kQWarp;
-            else if (flop <= BescE1Batch::kCap && lenA <= BescE1Batch::kAEntries) cls = kQE1;
-            else if (flop <= BescMidRank::kCap && lenA <= BescMidRank::kAEntries) cls = kQMid;
+            else if (flop <= warp_max) cls = flop <= kBatchQ256 ? kQ256 : kQ512;
+            else if (flop <= RankE1::kCap && lenA <= RankE1::kAEntries) cls = kQE1;
+            else if (flop <= RankMid::kCap && lenA <= RankMid::kAEntries) cls = kQMid;
             else cls = kQBeyond;
         }
 #pragma unroll
@@ -239,104 +234,47 @@ __global__ void __launch_bounds__(kBatchCountThreads) k_batch_count_rows(const S
     }
 }
 
-// Numeric persistent kernel of a warp queue (rows of at most 32*PMAX products): every warp
-// takes kBatchChunk rows per step through the queue's cursor until it is empty.
-template <int PMAX, typename T, typename KT>
-__global__ void __launch_bounds__(WsortShape<PMAX>::kThreads, WsortShape<PMAX>::kMinBlocks)
-    k_batch_warp_rows(const SpgemmArgs<T> *__restrict__ segs, const int *__restrict__ seg_row_base, int nseg,
+// Persistent kernel of a queue whose rows take rank shape Sh, one phase: every warp (or
+// CTA) takes rows through the queue's cursor until it is empty, warps kBatchChunk at a
+// time.  The symbolic phase writes each row's count to c_rpt.
+template <typename Sh, bool kNum, typename T>
+__global__ void __launch_bounds__(Sh::kThreads, Sh::kMinBlocks)
+    k_batch_rank_rows(const SpgemmArgs<T> *__restrict__ segs, const int *__restrict__ seg_row_base, int nseg,
                       const int *__restrict__ queue, const int *count, int *cursor)
 {
-    using Sh = WsortShape<PMAX>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ SpgemmArgs<T> s_segs[kBatchMaxSegs];
     __shared__ int s_base[kBatchMaxSegs + 1];
     batch_load_segs<T>(segs, seg_row_base, nseg, s_segs, s_base);
-    const int lane = lane_id();
-    const int warp = threadIdx.x >> 5;
-    const WsortSmem<PMAX, true, T, KT> sm(smem_raw + (size_t)warp * Sh::template per_warp<true, T, KT>());
     const int n = *count;
-    unsigned long long nnz_unused = 0;  // the counts were made by the symbolic phase
-    for (;;) {
-        int u0 = 0;
-        if (lane == 0) u0 = atomicAdd(cursor, kBatchChunk);
-        u0 = __shfl_sync(kFull, u0, 0);
-        if (u0 >= n) break;
-        const int u1 = min(n, u0 + kBatchChunk);
-        for (int u = u0; u < u1; ++u) {
-            const int gr = __ldg(queue + u);
-            const int s = batch_segment(s_base, nseg, gr);
-            wsort_process_row<PMAX, true, T, KT>(s_segs[s], gr - s_base[s], sm, nnz_unused);
+    unsigned long long nnz_unused = 0;  // the segments' totals come from their scans
+    int late_unused = 0;
+    auto row = [&](const RankSmem<Sh, T> &sm, int u) {
+        const int gr = __ldg(queue + u);
+        const int s = batch_segment(s_base, nseg, gr);
+        const SpgemmArgs<T> &g = s_segs[s];
+        rank_row<Sh, kNum, T>(g, gr - s_base[s], sm, rank_levels(g.N, Sh::kTop), nnz_unused, &late_unused);
+    };
+    if constexpr (Sh::kGroups > 1) {
+        const RankSmem<Sh, T> sm(smem_raw + (size_t)(threadIdx.x >> 5) * Sh::template group_bytes<kNum>());
+        for (;;) {
+            int u0 = 0;
+            if (lane_id() == 0) u0 = atomicAdd(cursor, kBatchChunk);
+            u0 = __shfl_sync(kFull, u0, 0);
+            if (u0 >= n) break;
+            const int u1 = min(n, u0 + kBatchChunk);
+            for (int u = u0; u < u1; ++u) row(sm, u);
         }
-    }
-}
-
-// Persistent kernel of a CTA queue (rows of at most Shape::kCap products), one phase:
-// every CTA takes one row per step through the queue's cursor until it is empty.  The
-// symbolic phase writes each row's count to c_rpt.
-template <typename Shape, bool kNum, typename T, typename KT>
-__global__ void __launch_bounds__(Shape::kThreads, Shape::kMinBlocks)
-    k_batch_cta_rows(const SpgemmArgs<T> *__restrict__ segs, const int *__restrict__ seg_row_base, int nseg,
-                     const int *__restrict__ queue, const int *count, int *cursor)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ SpgemmArgs<T> s_segs[kBatchMaxSegs];
-    __shared__ int s_base[kBatchMaxSegs + 1];
-    __shared__ int s_warp_sums[32];
-    __shared__ KT s_last[32];
-    __shared__ int s_unit;
-    __shared__ BescScratch s_sc;
-    if (threadIdx.x == 0) s_sc.reset();
-    batch_load_segs<T>(segs, seg_row_base, nseg, s_segs, s_base);
-    const BescSmem<Shape, kNum, KT, T> sm(smem_raw);
-    sm.init();
-    const int n = *count;
-    unsigned long long nnz_unused = 0;
-    for (;;) {
-        if (threadIdx.x == 0) s_unit = atomicAdd(cursor, 1);
-        __syncthreads();
-        const int u = s_unit;
-        __syncthreads();
-        if (u >= n) break;
-        const int gr = __ldg(queue + u);
-        const int s = batch_segment(s_base, nseg, gr);
-        besc_row<Shape, kNum, T, KT>(s_segs[s], gr - s_base[s], sm, s_warp_sums, s_last, &s_sc, nnz_unused);
-    }
-}
-
-// Symbolic persistent kernel of the kQMid queue: every CTA counts one row per cursor step
-// in a shared-memory hash table (EscMid's symbolic shape).
-static __global__ void __launch_bounds__(EscMid::kThreads, 1) k_batch_cta_count(const SpgemmArgs<double> *__restrict__ segs,
-                                                                        const int *__restrict__ seg_row_base,
-                                                                        int nseg, const int *__restrict__ queue,
-                                                                        const int *count, int *cursor)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ SpgemmArgs<double> s_segs[kBatchMaxSegs];
-    __shared__ int s_base[kBatchMaxSegs + 1];
-    __shared__ int s_warp_sums[32];
-    __shared__ int s_unit;
-    __shared__ int s_count;
-    batch_load_segs<double>(segs, seg_row_base, nseg, s_segs, s_base);
-    int *table = reinterpret_cast<int *>(smem_raw);
-    int *s_incl = table + EscMid::kTable;
-    int *s_b0 = s_incl + EscMid::kAEntries;
-    const int n = *count;
-    for (;;) {
-        if (threadIdx.x == 0) s_unit = atomicAdd(cursor, 1);
-        __syncthreads();
-        const int u = s_unit;
-        __syncthreads();
-        if (u >= n) break;
-        const int gr = __ldg(queue + u);
-        const int s = batch_segment(s_base, nseg, gr);
-        const SpgemmArgs<double> &g = s_segs[s];
-        const int r = gr - s_base[s];
-        const int a0 = __ldg(g.arpt + r);
-        const int lenA = __ldg(g.arpt + r + 1) - a0;
-        const int flop = esc_scan_row<EscMid::kThreads, double>(g, a0, lenA, s_incl, s_b0, s_warp_sums);
-        const int tot = esc_count_row<EscMid, double>(g, lenA, flop, table, s_incl, s_b0, &s_count);
-        if (threadIdx.x == 0) g.c_rpt[r] = tot;
-        __syncthreads();
+    } else {
+        __shared__ int s_unit;
+        const RankSmem<Sh, T> sm(smem_raw);
+        for (;;) {
+            if (threadIdx.x == 0) s_unit = atomicAdd(cursor, 1);
+            __syncthreads();
+            const int u = s_unit;
+            if (u >= n) break;
+            row(sm, u);  // ends with a barrier
+        }
     }
 }
 

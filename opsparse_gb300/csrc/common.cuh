@@ -19,33 +19,34 @@ enum RowClass : int {
     kClsR8 = 0,   // flop <= 8,  lenA <= 8  : 8 lanes per row, registers only
     kClsR16 = 1,  // flop <= 16, lenA <= 16 : 16 lanes per row
     kClsR32 = 2,  // flop <= 32, lenA <= 32 : one warp per row
-    kClsW = 3,    // flop <= 128            : one warp per row, register sort
-    kClsE1 = 4,   // flop <= 1024, lenA <= 1024   : warp sort, warp hash or CTA bitonic sort
-    kClsE2 = 5,   // flop <= 13312, lenA <= 2560  : CTA bitonic sort (<= 4096) or CTA radix sort
+    kClsW = 3,    // flop <= 128            : one warp per row, column rank
+    kClsE1 = 4,   // flop <= 1024, lenA <= 1024   : column rank (64 or 128 threads) or warp hash
+    kClsE2 = 5,   // flop <= 13312, lenA <= 2560  : column rank (512 or 1,024 threads)
     kClsD = 6,    // larger                 : whole-GPU stable radix sort (dense accumulator fallback)
     kNumClasses = 7
 };
 
 // Extra device lists after the kNumClasses class lists: the numeric re-binning of the E1
 // rows and the size split of the E2 rows.
-// The last three split the E1 rows of a one-pass call into those computed in the
-// counting phase (by warp sort, or expand/sort/compress above kE1OnePassFlopMax products)
-// and those left to two passes.
+// The last four split the E1 rows of a one-pass call into those computed in the counting
+// phase, by rank shape, and those left to two passes.
 enum : int {
-    kXlE1Sort = 0,
+    kXlE1Small = 0,     // numeric re-binning of the E1 rows (PickE1)
     kXlE1Hash = 1,
-    kXlE1Esc = 2,
-    kXlE2Mid = 3,
-    kXlE2Large = 4,
-    kXlE1One = 5,
-    kXlE1Two = 6,
-    kXlE1OneLarge = 7,
-    kNumExtraLists = 8
+    kXlE1Rank = 2,
+    kXlE1Half = 3,
+    kXlE2Mid = 4,       // E2 rows by size (PickE2)
+    kXlE2Large = 5,
+    kXlE1One = 6,       // E1 rows of a one-pass call (PickStaged)
+    kXlE1Two = 7,
+    kXlE1OneLarge = 8,
+    kXlE1OneHalf = 9,
+    kNumExtraLists = 10
 };
 constexpr int kNumLists = kNumClasses + kNumExtraLists;
 
 constexpr int kSmallFlopMax = 8;   // R8 rows: symbolic inside k_setup, numeric k_small_rows
-constexpr int kWarpFlopMax = 128;  // W rows: warp register sort of at most 128 products
+constexpr int kWarpFlopMax = 128;  // W rows: a warp ranks at most 128 products
 constexpr int kEsc1FlopMax = 1024;
 constexpr int kEsc1AMax = 1024;
 constexpr int kEsc2FlopMax = 13312;
@@ -59,9 +60,6 @@ constexpr int kBlockFoldMin = 2560;
 constexpr int kFoldBlocks = 32;
 static_assert(kBlockFoldMin >= kEsc2AMax && kBlockFoldMin >= kEsc1AMax && kBlockFoldMin >= 128,
               "entries of more than kBlockFoldMin products occur only in D rows");
-// E1 rows computed in the counting phase of a one-pass call: by warp sort up to this many
-// products, by CTA expand/sort/compress above; column-window rows (below) keep two passes
-constexpr int kE1OnePassFlopMax = 512;
 // Column-window rows: rows whose B rows are long (at least 16 products per A entry) and
 // whose products all fall within kWinBits consecutive columns (banded and stencil
 // matrices).  They fold many products per output: counted over a window bitmap, computed
@@ -89,25 +87,43 @@ enum : int {
     kErrBadColumn = 8,        // an input column index is outside [0, cols)
 };
 
+// Row sizes of the shapes that compute the E1 and E2 rows (rank.cuh).
+constexpr int kE1SmallMax = 256;
+constexpr int kE1HalfMax = 512;
+constexpr int kE2MidMax = 4096;
+constexpr int kE2MidAMax = 1280;
+
+// Row cursors of one phase's kernels (a CTA draws its next row from its kernel's cursor).
+struct RowCursors {
+    int e1_half;   // E1 rows of the 512-product shape
+    int e1;        // E1 rows of the 1,024-product shape
+    int mid;       // E2 rows of the mid shape
+    int large;     // E2 rows of the large shape
+};
+
 // Device-side counters of one SpGEMM call.  Lives in the handle's workspace.
 struct DevInfo {
-    int counts[kNumClasses];      // rows listed in each class
+    // zeroed together at the start of the numeric phase
     int flags;                    // kErr* bits
+    int split[4];                 // E1 rows re-binned for the numeric phase (PickE1)
+    RowCursors next_num;          // the numeric phase's row cursors
+    // zeroed with the rest at the start of the counting phase
+    RowCursors next_sym;          // the counting phase's row cursors
+    int counts[kNumClasses];      // rows listed in each class
     int max_flop;                 // clamped to INT_MAX
     unsigned long long total_flop;
     unsigned long long total_nnz;
-    int next[2][kNumClasses];     // dynamic row cursors of the [symbolic, numeric] kernels
-    int split[3];                 // E1 rows re-binned for the numeric phase: [warp sort, hash, expand/sort]
     int split2[2];                // E2 rows by size, fixed at the symbolic phase: [mid shape, large shape]
-    int next_mid[2];              // row cursor of the mid-shape E2 kernel [symbolic, numeric]
-    int split1[3];                // E1 rows of a one-pass call: [warp sort, two passes, expand/sort/compress]
+    int split1[4];                // E1 rows of a one-pass call (PickStaged)
     unsigned long long staged_flop;  // products of the rows a one-pass call may stage
     int e1_one;                   // E1 rows a one-pass call may stage
+    int e1_size[3];               // E1 rows of at most 256, 512 and 1,024 products
+    int e2_size[2];               // E2 rows of the mid and the large shape
     unsigned long long d_len_a;   // A entries of the D rows
     unsigned long long d_flop;    // products of the D rows
     int d_cursor;                 // long runs listed by the D-row short-run fold
-    int rank_rows[3];             // CTA expand rows by the column-window rank path: [no late
-                                  // products, late products re-folded, too many late: sorted]
+    int rank_rows[3];             // E1 rows of the 1,024-product shape where B has at most 65,536
+                                  // columns, by products in repeated columns: [0, 1..128, more]
 };
 
 // Arguments shared by every SpGEMM kernel.

@@ -96,6 +96,7 @@ struct ops_handle_s {
     int plan_M = 0, plan_K = 0, plan_N = 0;
     const int *plan_arpt = nullptr, *plan_acol = nullptr, *plan_brpt = nullptr, *plan_bcol = nullptr;
     int counts[kNumClasses] = {};
+    int e1_size[3] = {}, e2_size[2] = {};  // E1 and E2 rows by shape (DevInfo)
     long long plan_flop = 0;
     long long plan_nnz = 0;
     int d_rows_path[2] = {};      // D rows of the last phase by [whole-GPU sort, dense kernel]

@@ -11,7 +11,7 @@
 //                         de-duplication, no table, no sort pass).
 //   k_warp_rows        <- k_*_shared_hash_tb for the small bins (symbolic.cuh:74-130,
 //                         numeric.cuh:109-205): one warp per row, table in shared memory.
-//   k_esc_rows (esc.cuh) <- the same kernels for the middle/large bins and
+//   k_rank_rows (rank.cuh) <- the same kernels for the small to large bins and
 //                         k_*_max_shared_hash_tb (symbolic.cuh:132-261, numeric.cuh:207-302).
 //   k_dense_rows       <- the global-hash fallback (symbolic.cuh:263-325, numeric.cuh:304-393):
 //                         one CTA per row over a dense accumulator and bitmap in HBM, which
@@ -56,66 +56,6 @@ __device__ __forceinline__ void block_add_u64(unsigned long long v, unsigned lon
     __syncthreads();
 }
 
-constexpr int kFoldUnroll = 4;  // fold steps whose operands are loaded together
-
-// Folds the runs [hs, he) owned by the calling thread (run h covers the sorted positions
-// [head(h), end(h)); runs of skip_len or more products are left to the caller): the
-// concatenation of the runs is walked one product per step, the operands of kFoldUnroll
-// steps loaded together (load(t, a, b, k) gives product t's operands and its B index),
-// and each completed run is passed to write(h, t, k, s) with one of its positions and B
-// indices.  A warp-wide FP64 FMA costs the same however few lanes are active, so packing
-// the steps makes a warp issue about as many FMAs as its busiest lane has products,
-// where one run per lane per step would issue kFoldUnroll per run.
-template <typename T, typename Head, typename End, typename Load, typename Write>
-__device__ __forceinline__ void fold_own_runs(int hs, int he, int skip_len, Head head, End end, Load load,
-                                              Write write)
-{
-    using AccT = Acc<T>;
-    using S = typename AccT::S;
-    int h = hs, t = 0, e = 0;  // current run, next position, end of the run
-    auto next_run = [&]() {    // from run h on: the first run to fold, or h == he
-        for (; h < he; ++h) {
-            t = head(h);
-            e = end(h);
-            if (e - t < skip_len) return;
-        }
-    };
-    next_run();
-    S s = AccT::zero();
-    while (h < he) {
-        T av[kFoldUnroll], bv[kFoldUnroll];
-        int hu[kFoldUnroll], pu[kFoldUnroll], ku[kFoldUnroll];
-#pragma unroll
-        for (int u = 0; u < kFoldUnroll; ++u) {
-            hu[u] = -1;
-            pu[u] = 0;
-            ku[u] = 0;
-            av[u] = T(0);
-            bv[u] = T(0);
-            if (h < he) {
-                hu[u] = h;
-                pu[u] = t;
-                load(t, av[u], bv[u], ku[u]);
-                if (++t == e) {
-                    ++h;
-                    next_run();
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kFoldUnroll; ++u) {
-            if (hu[u] >= 0) {
-                s = AccT::step(s, av[u], bv[u]);
-                const int hn = u + 1 < kFoldUnroll ? hu[u + 1] : (h < he ? h : -1);
-                if (hn != hu[u]) {  // run hu[u] is complete
-                    write(hu[u], pu[u], ku[u], s);
-                    s = AccT::zero();
-                }
-            }
-        }
-    }
-}
-
 // ==================================================================================
 // Setup: per-row product count, validation of A's columns, class assignment, and the
 // scatter of row ids into per-class lists (lists[c * M + i]).  One thread per row for
@@ -138,6 +78,7 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
     __shared__ unsigned long long s_flop[kSetupThreads / 32];
     __shared__ unsigned long long s_sflop[kSetupThreads / 32];
     __shared__ int s_e1one;
+    __shared__ int s_size[5];
     __shared__ unsigned s_small[kSetupThreads / 32];
     __shared__ int s_flags;
     const int lane = lane_id();
@@ -146,6 +87,7 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
     if (threadIdx.x == 0) {
         s_flags = 0;
         s_e1one = 0;
+        for (int i = 0; i < 5; ++i) s_size[i] = 0;
     }
     __syncthreads();
 
@@ -260,8 +202,10 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
             cls = kClsW;
         } else if (flop <= th.e1 && lenA <= kEsc1AMax) {
             cls = kClsE1;
+            atomicAdd(&s_size[flop <= kE1SmallMax ? 0 : (flop <= kE1HalfMax ? 1 : 2)], 1);
         } else if (flop <= th.e2 && lenA <= kEsc2AMax) {
             cls = kClsE2;
+            atomicAdd(&s_size[flop <= kE2MidMax && lenA <= kE2MidAMax ? 3 : 4], 1);
         } else {
             cls = kClsD;
             atomicAdd(&info->d_len_a, (unsigned long long)lenA);
@@ -338,6 +282,8 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
         for (int w = 0; w < kSetupThreads / 32; ++w) ts += s_sflop[w];
         if (ts) atomicAdd(&info->staged_flop, ts);
         if (s_e1one) atomicAdd(&info->e1_one, s_e1one);
+        for (int i = 0; i < 5; ++i)
+            if (s_size[i]) atomicAdd(i < 3 ? &info->e1_size[i] : &info->e2_size[i - 3], s_size[i]);
         unsigned long long sn = 0;
         for (int w = 0; w < kSetupThreads / 32; ++w) sn += s_small[w];
         if (sn) atomicAdd(&info->total_nnz, sn);

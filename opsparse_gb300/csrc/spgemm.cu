@@ -18,13 +18,13 @@
 
 #include <algorithm>
 #include <array>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <new>
 #include <string>
 
-#include "besc.cuh"
-#include "wsort.cuh"
+#include "lists.cuh"
 #include "internal.hpp"
 #include "opsparse_gb300.h"
 
@@ -43,45 +43,34 @@ struct Mat {
     const void *val;
 };
 
-template <typename Shape, typename T>
-void set_besc_attrs()
+template <typename Sh, typename T>
+void set_rank_attrs()
 {
-    cudaFuncSetAttribute(k_besc_rows<Shape, true, T, unsigned>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)Shape::template smem<true, unsigned, T>());
-    cudaFuncSetAttribute(k_besc_rows<Shape, true, T, unsigned long long>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)Shape::template smem<true, unsigned long long, T>());
-    cudaFuncSetAttribute(k_besc_rows<Shape, false, T, unsigned>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)Shape::template smem<false, unsigned, T>());
+    cudaFuncSetAttribute(k_rank_rows<Sh, true, T, Sh::kCap == RankE1::kCap>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)Sh::template smem<true>());
+    cudaFuncSetAttribute(k_rank_rows<Sh, false, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)Sh::template smem<false>());
 }
 
-// Launch the CTA-per-row bitonic kernel of `Shape` on `s`: numeric keys pack the product
-// index below the column and need 64 bits when the two do not fit in 32.
-template <typename Shape, bool kNum, typename T>
-void launch_besc(const SpgemmArgs<T> &g, const int *list, const int *count_ptr, int *cursor, int grid,
+// Launch the rank kernel of shape Sh for at most n listed rows (the exact count is on the
+// device).  The E1 shape counts its rows by late products.
+template <typename Sh, bool kNum, typename T>
+void launch_rank(ops_handle_s *h, const SpgemmArgs<T> &g, const int *list, const int *count_ptr, int *cursor, int n,
                  cudaStream_t s)
 {
-    if (!kNum) {
-        k_besc_rows<Shape, false, T, unsigned>
-            <<<grid, Shape::kThreads, Shape::template smem<false, unsigned, T>(), s>>>(g, list, count_ptr, cursor);
-    } else if (ceil_log2(std::max(g.N, 2)) + Shape::kIdBits <= 32) {
-        k_besc_rows<Shape, true, T, unsigned>
-            <<<grid, Shape::kThreads, Shape::template smem<true, unsigned, T>(), s>>>(g, list, count_ptr, cursor);
-    } else {
-        k_besc_rows<Shape, true, T, unsigned long long>
-            <<<grid, Shape::kThreads, Shape::template smem<true, unsigned long long, T>(), s>>>(g, list, count_ptr,
-                                                                                             cursor);
-    }
-}
-
-// The E1 expand rows' numeric kernel: the rank shape where B has at most kRankWinBits
-// columns (every row fits the window), else the sort-only shape, whose smaller shared
-// memory keeps one more CTA per SM for rows that could not take the rank path.
-template <typename T>
-void launch_besc_e1(const SpgemmArgs<T> &g, const int *list, const int *count_ptr, int *cursor, int grid,
-                    cudaStream_t s)
-{
-    if (g.N <= kRankWinBits) launch_besc<BescE1, true, T>(g, list, count_ptr, cursor, grid, s);
-    else launch_besc<BescE1Sort, true, T>(g, list, count_ptr, cursor, grid, s);
+    if (n <= 0) return;
+    // one wave of CTAs that stay until the list is empty, or beside D rows as many as take
+    // rank_rows_per_group rows each
+    constexpr int by_smem = (int)(227 * 1024 / (Sh::template smem<kNum>() + 1024));
+    constexpr int ctas = by_smem < Sh::kMinBlocks ? by_smem : Sh::kMinBlocks;
+    static_assert(ctas >= 1, "a CTA fits an SM");
+    constexpr int per_cta = Sh::kGroups * rank_rows_per_group<Sh>();
+    const int wave = std::min((n + Sh::kGroups - 1) / Sh::kGroups, h->num_sms * ctas);
+    const bool beside_d = h->counts[kClsD] > 0;
+    const int grid = beside_d ? std::max(wave, (n + per_cta - 1) / per_cta) : wave;
+    k_rank_rows<Sh, kNum, T, kNum && Sh::kCap == RankE1::kCap><<<grid, Sh::kThreads, Sh::template smem<kNum>(), s>>>(
+        g, list, count_ptr, cursor, beside_d ? rank_rows_per_group<Sh>() : INT_MAX);
+    ++h->launches;
 }
 
 template <typename T>
@@ -89,26 +78,14 @@ void set_smem_attrs()
 {
     cudaFuncSetAttribute(k_warp_rows<true, T, 2 * kSplitNnz>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)warp_rows_smem<true, T, 2 * kSplitNnz>());
-    cudaFuncSetAttribute(k_esc_rows<EscLarge, true, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)EscLarge::kNumericSmem);
-    cudaFuncSetAttribute(k_esc_rows<EscLarge, false, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)EscLarge::kSymbolicSmem);
-    cudaFuncSetAttribute(k_esc_rows<EscMid, false, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)EscMid::kSymbolicSmem);
     cudaFuncSetAttribute(k_warp_rows<false, T, 2 * kEsc1FlopMax>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)warp_rows_smem<false, T, 2 * kEsc1FlopMax>());
-    set_besc_attrs<BescE1, T>();
-    set_besc_attrs<BescE1Sort, T>();
-    set_besc_attrs<BescMid, T>();
-    cudaFuncSetAttribute(k_wsort_rows<4, true, T, unsigned>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)WsortShape<4>::smem<true, T, unsigned>());
-    cudaFuncSetAttribute(k_wsort_rows<4, true, T, unsigned long long>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)WsortShape<4>::smem<true, T, unsigned long long>());
-    cudaFuncSetAttribute(k_wsort_rows<16, true, T, unsigned>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)WsortShape<16>::smem<true, T, unsigned>());
-    cudaFuncSetAttribute(k_wsort_rows<16, true, T, unsigned long long>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)WsortShape<16>::smem<true, T, unsigned long long>());
+    set_rank_attrs<RankW, T>();
+    set_rank_attrs<RankS, T>();
+    set_rank_attrs<RankM, T>();
+    set_rank_attrs<RankE1, T>();
+    set_rank_attrs<RankMid, T>();
+    set_rank_attrs<RankLarge, T>();
 }
 
 int ensure_ws(ops_handle_s *h, int M, cudaStream_t st)
@@ -116,8 +93,7 @@ int ensure_ws(ops_handle_s *h, int M, cudaStream_t st)
     if (h->ws && h->ws_M >= M) return OPS_OK;
     size_t cub_bytes = 0;
     OPS_CUDA(h, cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, (int *)nullptr, (int *)nullptr, M + 1, st));
-    // one list per class, three for the numeric re-binning of E1 rows and two for the
-    // E2 rows by size
+    // one list per class and the extra lists of re-binned classes
     const size_t lists_b = align_up(sizeof(int) * (size_t)(kNumLists) * (size_t)M, 256);
     const size_t flop_b = align_up(sizeof(int) * (size_t)M, 256);
     const size_t soff_b = align_up(sizeof(int) * ((size_t)M + 1), 256);
@@ -256,35 +232,27 @@ int launch_staged_class(ops_handle_s *h, const GA &gs, int c, const int *list, i
         case kClsR32:
             k_reg_rows<32, true, T><<<grid_for(n, 8, sms * 8), 256, 0, s>>>(g, list, n);
             break;
-        case kClsW: {
-            using Sh = WsortShape<4>;
-            const int grid = grid_for(n, Sh::kWarps, sms * 8);
-            if (g.N <= (1 << (32 - Sh::kIdBits))) {
-                k_wsort_rows<4, true, T, unsigned>
-                    <<<grid, Sh::kThreads, Sh::smem<true, T, unsigned>(), s>>>(g, list, &h->info->counts[c]);
-            } else {
-                k_wsort_rows<4, true, T, unsigned long long>
-                    <<<grid, Sh::kThreads, Sh::smem<true, T, unsigned long long>(), s>>>(g, list, &h->info->counts[c]);
-            }
+        case kClsW:
+            launch_rank<RankW, true, T>(h, g, list, &h->info->counts[c], nullptr, n, s);
             break;
-        }
         case kClsE1: {
-            // the staged rows (not column-window rows) into the staging area: by warp sort
-            // up to kE1OnePassFlopMax products, else (on an extra stream) by CTA
-            // expand/sort/compress; the rest counted by the warp hash
+            // the staged rows (not column-window rows) into the staging area by rank shape,
+            // the larger shapes on an extra stream; the rest counted by the warp hash
             int *one = xl + kXlE1One * M;
             int *two = xl + kXlE1Two * M;
             int *one_large = xl + kXlE1OneLarge * M;
-            k_split_list<3, PickStaged><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
+            int *one_half = xl + kXlE1OneHalf * M;
+            k_split_list<4, PickStaged><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
                 list, &h->info->counts[c], PickStaged{h->soff, g.row_flop}, one, (int)M, h->info->split1);
             OPS_CUDA(h, cudaGetLastError());
             ++h->launches;
             OPS_CUDA(h, cudaEventRecord(h->ev_x_fork[0], s));
             OPS_CUDA(h, cudaStreamWaitEvent(h->side_x[0], h->ev_x_fork[0], 0));
-            launch_besc_e1<T>(g, one_large, &h->info->split1[2], &h->info->next[0][c], std::min(n, sms * 8),
-                              h->side_x[0]);
+            launch_rank<RankE1, true, T>(h, g, one_large, &h->info->split1[2], &h->info->next_sym.e1, h->e1_size[2],
+                                         h->side_x[0]);
+            launch_rank<RankM, true, T>(h, g, one_half, &h->info->split1[3], &h->info->next_sym.e1_half, h->e1_size[1],
+                                        h->side_x[0]);
             OPS_CUDA(h, cudaGetLastError());
-            ++h->launches;
             SpgemmArgs<double> gc{};
             gc.arpt = g.arpt;
             gc.acol = g.acol;
@@ -296,21 +264,15 @@ int launch_staged_class(ops_handle_s *h, const GA &gs, int c, const int *list, i
             gc.row_flop = g.row_flop;
             gc.c_rpt = g.c_rpt;
             gc.info = g.info;
-            k_warp_rows<false, double, 2 * kEsc1FlopMax>
-                <<<grid_for(n, kWarpRowsThreads / 32, sms * 3), kWarpRowsThreads,
-                   warp_rows_smem<false, double, 2 * kEsc1FlopMax>(), h->side_x[0]>>>(gc, two, &h->info->split1[1]);
-            OPS_CUDA(h, cudaGetLastError());
-            ++h->launches;
-            OPS_CUDA(h, cudaEventRecord(h->ev_x_join[0], h->side_x[0]));
-            using Sh = WsortShape<16>;
-            const int sgrid = grid_for(n, Sh::kWarps, sms * 4);
-            if (g.N <= (1 << (32 - Sh::kIdBits))) {
-                k_wsort_rows<16, true, T, unsigned>
-                    <<<sgrid, Sh::kThreads, Sh::smem<true, T, unsigned>(), s>>>(g, one, &h->info->split1[0]);
-            } else {
-                k_wsort_rows<16, true, T, unsigned long long>
-                    <<<sgrid, Sh::kThreads, Sh::smem<true, T, unsigned long long>(), s>>>(g, one, &h->info->split1[0]);
+            if (!h->stage_e1_all) {
+                k_warp_rows<false, double, 2 * kEsc1FlopMax>
+                    <<<grid_for(n, kWarpRowsThreads / 32, sms * 3), kWarpRowsThreads,
+                       warp_rows_smem<false, double, 2 * kEsc1FlopMax>(), h->side_x[0]>>>(gc, two, &h->info->split1[1]);
+                OPS_CUDA(h, cudaGetLastError());
+                ++h->launches;
             }
+            OPS_CUDA(h, cudaEventRecord(h->ev_x_join[0], h->side_x[0]));
+            launch_rank<RankS, true, T>(h, g, one, &h->info->split1[0], nullptr, h->e1_size[0], s);
             OPS_CUDA(h, cudaGetLastError());
             OPS_CUDA(h, cudaStreamWaitEvent(s, h->ev_x_join[0], 0));
             break;
@@ -325,23 +287,21 @@ int launch_staged_class(ops_handle_s *h, const GA &gs, int c, const int *list, i
             ++h->launches;
             OPS_CUDA(h, cudaEventRecord(h->ev_x_fork[1], s));
             OPS_CUDA(h, cudaStreamWaitEvent(h->side_x[1], h->ev_x_fork[1], 0));
-            if (n > 1) {
+            if (h->e2_size[1] > 1) {
                 k_sort_heavy_first<<<1, 1024, 0, h->side_x[1]>>>(large_list, &h->info->split2[1], h->row_flop);
                 OPS_CUDA(h, cudaGetLastError());
                 ++h->launches;
             }
-            k_esc_rows<EscLarge, true, T><<<std::min(n, sms), EscLarge::kThreads, EscLarge::kNumericSmem,
-                                            h->side_x[1]>>>(g, large_list, &h->info->split2[1], &h->info->next[0][c]);
+            launch_rank<RankLarge, true, T>(h, g, large_list, &h->info->split2[1], &h->info->next_sym.large,
+                                            h->e2_size[1], h->side_x[1]);
             OPS_CUDA(h, cudaGetLastError());
-            ++h->launches;
             OPS_CUDA(h, cudaEventRecord(h->ev_x_join[1], h->side_x[1]));
-            if (n > 1) {
+            if (h->e2_size[0] > 1) {
                 k_sort_heavy_first<<<1, 1024, 0, s>>>(mid_list, &h->info->split2[0], h->row_flop);
                 OPS_CUDA(h, cudaGetLastError());
                 ++h->launches;
             }
-            launch_besc<BescMid, true, T>(g, mid_list, &h->info->split2[0], &h->info->next_mid[0],
-                                          std::min(n, sms * 4), s);
+            launch_rank<RankMid, true, T>(h, g, mid_list, &h->info->split2[0], &h->info->next_sym.mid, h->e2_size[0], s);
             OPS_CUDA(h, cudaGetLastError());
             OPS_CUDA(h, cudaStreamWaitEvent(s, h->ev_x_join[1], 0));
             break;
@@ -475,22 +435,9 @@ int launch_classes(ops_handle_s *h, const SpgemmArgs<T> &g, cudaStream_t st)
             case kClsR32:
                 k_reg_rows<32, kNum, T><<<grid_for(n, 8, sms * 8), 256, 0, s>>>(g, list, n);
                 break;
-            case kClsW: {  // warp sort: products sorted in registers, no table
-                using Sh = WsortShape<4>;
-                const int grid = grid_for(n, Sh::kWarps, sms * 8);
-                if (!kNum) {
-                    k_wsort_rows<4, false, T, unsigned>
-                        <<<grid, Sh::kThreads, Sh::smem<false, T, unsigned>(), s>>>(g, list, &h->info->counts[c]);
-                } else if (g.N <= (1 << (32 - Sh::kIdBits))) {
-                    k_wsort_rows<4, true, T, unsigned>
-                        <<<grid, Sh::kThreads, Sh::smem<true, T, unsigned>(), s>>>(g, list, &h->info->counts[c]);
-                } else {
-                    k_wsort_rows<4, true, T, unsigned long long>
-                        <<<grid, Sh::kThreads, Sh::smem<true, T, unsigned long long>(), s>>>(g, list,
-                                                                                            &h->info->counts[c]);
-                }
+            case kClsW:
+                launch_rank<RankW, kNum, T>(h, g, list, &h->info->counts[c], nullptr, n, s);
                 break;
-            }
             case kClsE1: {
                 if (!kNum) {  // distinct-column count: one warp per row, table of 2*flop slots
                     k_warp_rows<false, T, 2 * kEsc1FlopMax>
@@ -498,46 +445,38 @@ int launch_classes(ops_handle_s *h, const SpgemmArgs<T> &g, cudaStream_t st)
                            warp_rows_smem<false, T, 2 * kEsc1FlopMax>(), s>>>(g, list, &h->info->counts[c]);
                     break;
                 }
-                // re-bin by output size: warp sort / warp hash on this stream,
-                // expand/sort/compress on an extra stream (a one-pass call re-bins only
+                // re-bin by output size: the warp's rank shape and warp hash on this stream,
+                // the larger rank shapes on an extra stream (a one-pass call re-bins only
                 // the rows it left to two passes)
-                int *sort_list = xl + kXlE1Sort * M;
+                int *small_list = xl + kXlE1Small * M;
+                int *half_list = xl + kXlE1Half * M;
                 int *hash_list = xl + kXlE1Hash * M;
-                int *esc_list = xl + kXlE1Esc * M;
+                int *rank_list = xl + kXlE1Rank * M;
                 const int *e1_list = staged ? xl + kXlE1Two * M : list;
                 const int *e1_count = staged ? &h->info->split1[1] : &h->info->counts[c];
-                k_split_list<3, PickE1><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
-                    e1_list, e1_count, PickE1{g.c_rpt, g.row_flop, kWsortFlopMax}, sort_list, (int)M,
-                    h->info->split);
+                k_split_list<4, PickE1><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
+                    e1_list, e1_count, PickE1{g.c_rpt, g.row_flop}, small_list, (int)M, h->info->split);
                 OPS_CUDA(h, cudaGetLastError());
                 ++h->launches;
                 cudaStream_t sx = fork_x(0, s);
                 if (!sx) return fail(h, OPS_CUDA_ERROR, "stream fork failed");
-                launch_besc_e1<T>(g, esc_list, &h->info->split[2], &h->info->next[1][c], std::min(n, sms * 8), sx);
+                launch_rank<RankE1, true, T>(h, g, rank_list, &h->info->split[2], &h->info->next_num.e1, h->e1_size[2],
+                                             sx);
+                launch_rank<RankM, true, T>(h, g, half_list, &h->info->split[3], &h->info->next_num.e1_half,
+                                            h->e1_size[1], sx);
                 OPS_CUDA(h, cudaGetLastError());
-                ++h->launches;
                 if (!join_x(0, s)) return fail(h, OPS_CUDA_ERROR, "stream join failed");
-                using Sh = WsortShape<16>;
-                const int sgrid = grid_for(n, Sh::kWarps, sms * 4);
-                if (g.N <= (1 << (32 - Sh::kIdBits))) {
-                    k_wsort_rows<16, true, T, unsigned>
-                        <<<sgrid, Sh::kThreads, Sh::smem<true, T, unsigned>(), s>>>(g, sort_list, &h->info->split[0]);
-                } else {
-                    k_wsort_rows<16, true, T, unsigned long long>
-                        <<<sgrid, Sh::kThreads, Sh::smem<true, T, unsigned long long>(), s>>>(g, sort_list,
-                                                                                              &h->info->split[0]);
-                }
+                launch_rank<RankS, true, T>(h, g, small_list, &h->info->split[0], nullptr, h->e1_size[0], s);
                 OPS_CUDA(h, cudaGetLastError());
-                ++h->launches;
                 k_warp_rows<true, T, 2 * kSplitNnz>
                     <<<grid_for(n, kWarpRowsThreads / 32, sms * 4), kWarpRowsThreads,
                        warp_rows_smem<true, T, 2 * kSplitNnz>(), s>>>(g, hash_list, &h->info->split[1]);
                 break;
             }
             case kClsE2: {
-                // mid shape (3 CTAs per SM) on this stream, large shape (1 per SM) on an
-                // extra stream; the split and the longest-first order are made once, by
-                // the symbolic phase, and reused by numeric
+                // mid shape on this stream, large shape (one CTA per SM) on an extra stream;
+                // the split and the longest-first order are made once, by the symbolic
+                // phase, and reused by numeric
                 int *mid_list = xl + kXlE2Mid * M;
                 int *large_list = xl + kXlE2Large * M;
                 if (!kNum) {
@@ -548,31 +487,21 @@ int launch_classes(ops_handle_s *h, const SpgemmArgs<T> &g, cudaStream_t st)
                 }
                 cudaStream_t sx = fork_x(1, s);
                 if (!sx) return fail(h, OPS_CUDA_ERROR, "stream fork failed");
-                if (!kNum && n > 1) {
+                if (!kNum && h->e2_size[1] > 1) {
                     k_sort_heavy_first<<<1, 1024, 0, sx>>>(large_list, &h->info->split2[1], h->row_flop);
                     OPS_CUDA(h, cudaGetLastError());
                     ++h->launches;
                 }
-                // large rows: radix-sort expand/sort/compress (for 8K-16K products the
-                // 3 radix passes beat a 16K-key bitonic network); counting by hash table
-                k_esc_rows<EscLarge, kNum, T>
-                    <<<std::min(n, sms), EscLarge::kThreads, kNum ? EscLarge::kNumericSmem : EscLarge::kSymbolicSmem,
-                       sx>>>(g, large_list, &h->info->split2[1], &h->info->next[kNum][c]);
+                RowCursors &next = kNum ? h->info->next_num : h->info->next_sym;
+                launch_rank<RankLarge, kNum, T>(h, g, large_list, &h->info->split2[1], &next.large, h->e2_size[1], sx);
                 OPS_CUDA(h, cudaGetLastError());
-                ++h->launches;
                 if (!join_x(1, s)) return fail(h, OPS_CUDA_ERROR, "stream join failed");
-                if (!kNum && n > 1) {
+                if (!kNum && h->e2_size[0] > 1) {
                     k_sort_heavy_first<<<1, 1024, 0, s>>>(mid_list, &h->info->split2[0], h->row_flop);
                     OPS_CUDA(h, cudaGetLastError());
                     ++h->launches;
                 }
-                if (kNum) {  // mid rows: bitonic expand/sort/compress
-                    launch_besc<BescMid, true, T>(g, mid_list, &h->info->split2[0], &h->info->next_mid[1],
-                                                  std::min(n, sms * 4), s);
-                } else {  // counting by hash table
-                    k_esc_rows<EscMid, false, T><<<std::min(n, sms * 4), EscMid::kThreads, EscMid::kSymbolicSmem, s>>>(
-                        g, mid_list, &h->info->split2[0], &h->info->next_mid[0]);
-                }
+                launch_rank<RankMid, kNum, T>(h, g, mid_list, &h->info->split2[0], &next.mid, h->e2_size[0], s);
                 break;
             }
             case kClsD: {
@@ -675,6 +604,8 @@ int run_symbolic(ops_handle_s *h, const Mat &A, const Mat &B, int *c_rpt, long l
     if (hi.flags & kErrRowFlopOverflow)
         return fail(h, OPS_INT32_OVERFLOW, "a row of C has more than INT32_MAX intermediate products");
     std::memcpy(h->counts, hi.counts, sizeof(h->counts));
+    std::memcpy(h->e1_size, hi.e1_size, sizeof(h->e1_size));
+    std::memcpy(h->e2_size, hi.e2_size, sizeof(h->e2_size));
     h->plan_th = h->th;
     h->plan_M = M;
     h->plan_K = A.cols;
@@ -729,10 +660,7 @@ int run_numeric(ops_handle_s *h, const Mat &A, const Mat &B, const int *c_rpt, i
     if (!h->plan_valid || h->plan_M != A.rows || h->plan_K != A.cols || h->plan_N != B.cols ||
         h->plan_arpt != A.rpt || h->plan_acol != A.col || h->plan_brpt != B.rpt || h->plan_bcol != B.col)
         return fail(h, OPS_NOT_SUPPORTED, "numeric phase without a matching symbolic phase on this handle");
-    OPS_CUDA(h, cudaMemsetAsync(&h->info->flags, 0, sizeof(int), st));
-    OPS_CUDA(h, cudaMemsetAsync(h->info->next[1], 0, sizeof(h->info->next[1]), st));
-    OPS_CUDA(h, cudaMemsetAsync(h->info->split, 0, sizeof(h->info->split), st));
-    OPS_CUDA(h, cudaMemsetAsync(&h->info->next_mid[1], 0, sizeof(int), st));
+    OPS_CUDA(h, cudaMemsetAsync(h->info, 0, offsetof(DevInfo, next_sym), st));
     SpgemmArgs<T> g{};
     g.arpt = A.rpt;
     g.acol = A.col;
@@ -1017,7 +945,7 @@ int ops_handle_subclass_rows(ops_handle_t h, int32_t *out, int n)
         DevInfo d{};
         OPS_CUDA(h, cudaMemcpy(&d, h->info, sizeof(DevInfo), cudaMemcpyDeviceToHost));
         // a one-pass call computes its staged E1 rows while counting (split1)
-        v[0] = d.split[0] + d.split1[0];
+        v[0] = d.split[0] + d.split[3] + d.split1[0] + d.split1[3];
         v[1] = d.split[1];
         v[2] = d.split[2] + d.split1[2];
         v[3] = d.split2[0];
