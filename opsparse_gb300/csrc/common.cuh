@@ -99,6 +99,7 @@ struct RowCursors {
     int e1;        // E1 rows of the 1,024-product shape
     int mid;       // E2 rows of the mid shape
     int large;     // E2 rows of the large shape
+    int group;     // groups of rows of one pattern
 };
 
 // Device-side counters of one SpGEMM call.  Lives in the handle's workspace.
@@ -119,6 +120,8 @@ struct DevInfo {
     int e1_one;                   // E1 rows a one-pass call may stage
     int e1_size[3];               // E1 rows of at most 256, 512 and 1,024 products
     int e2_size[2];               // E2 rows of the mid and the large shape
+    int e1_chain;                 // E1 rows whose A row the next row of A repeats, moved by one column
+    int groups;                   // groups of rows of one pattern (regular.cuh)
     unsigned long long d_len_a;   // A entries of the D rows
     unsigned long long d_flop;    // products of the D rows
     int d_cursor;                 // long runs listed by the D-row short-run fold

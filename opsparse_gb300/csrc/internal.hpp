@@ -61,6 +61,10 @@ struct ops_handle_s {
     int ws_M = -1;
     int *lists = nullptr;
     int *row_flop = nullptr;
+    unsigned char *link = nullptr;   // [M] link flags of the rows
+    int2 *groups = nullptr;          // groups of rows of one pattern: (first row, rows)
+    unsigned char *b_link = nullptr; // [b_link_rows] B's part of the links (grow-only)
+    long long b_link_rows = 0;
     DevInfo *info = nullptr;
     void *cub_tmp = nullptr;
     size_t cub_bytes = 0;
@@ -97,6 +101,7 @@ struct ops_handle_s {
     const int *plan_arpt = nullptr, *plan_acol = nullptr, *plan_brpt = nullptr, *plan_bcol = nullptr;
     int counts[kNumClasses] = {};
     int e1_size[3] = {}, e2_size[2] = {};  // E1 and E2 rows by shape (DevInfo)
+    bool regular = false;         // some E1 rows are in groups of one pattern (regular.cuh)
     long long plan_flop = 0;
     long long plan_nnz = 0;
     int d_rows_path[2] = {};      // D rows of the last phase by [whole-GPU sort, dense kernel]

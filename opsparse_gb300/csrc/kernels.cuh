@@ -70,7 +70,8 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
                                                         const int *__restrict__ brpt, const int *__restrict__ bcol,
                                                         int M, int K, int N, int *__restrict__ row_flop,
                                                         int *__restrict__ lists, int *__restrict__ c_rownnz,
-                                                        int *__restrict__ sflop, DevInfo *info, Thresholds th)
+                                                        int *__restrict__ sflop, unsigned char *__restrict__ link,
+                                                        DevInfo *info, Thresholds th)
 {
     static_assert(kSmallFlopMax == kSetupUnroll, "R8 rows are gathered from the light-row registers");
     __shared__ int s_cnt[kNumClasses];
@@ -79,6 +80,7 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
     __shared__ unsigned long long s_sflop[kSetupThreads / 32];
     __shared__ int s_e1one;
     __shared__ int s_size[5];
+    __shared__ int s_chained;
     __shared__ unsigned s_small[kSetupThreads / 32];
     __shared__ int s_flags;
     const int lane = lane_id();
@@ -87,18 +89,22 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
     if (threadIdx.x == 0) {
         s_flags = 0;
         s_e1one = 0;
+        s_chained = 0;
         for (int i = 0; i < 5; ++i) s_size[i] = 0;
     }
     __syncthreads();
 
     const int r = blockIdx.x * kSetupThreads + threadIdx.x;
     const bool in = r < M;
-    int a0 = 0, a1 = 0;
+    int a0 = 0, a1 = 0, a2 = 0;
     if (in) {
         a0 = arpt[r];
         a1 = arpt[r + 1];
+        a2 = r + 1 < M ? arpt[r + 2] : a1;
     }
     const int lenA = a1 - a0;
+    bool windowed = false;  // a heavy row's products fall within kWinBits columns
+    bool chained = false;   // the next row of A is this one moved by one column
     long long flop = 0;
     bool bad = false;
     const bool light = in && lenA <= kSetupUnroll;
@@ -128,14 +134,13 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
         const int h1 = __shfl_sync(kFull, a1, t);
         unsigned long long s = 0;
         bool hb = false;
+        int jj[kSetupUnroll], lo[kSetupUnroll], hi[kSetupUnroll];
         for (int p0 = h0; p0 < h1; p0 += 32 * kSetupUnroll) {
-            int jj[kSetupUnroll];
 #pragma unroll
             for (int u = 0; u < kSetupUnroll; ++u) {
                 const int p = p0 + u * 32 + lane;
                 jj[u] = p < h1 ? __ldg(acol + p) : -1;
             }
-            int lo[kSetupUnroll], hi[kSetupUnroll];
 #pragma unroll
             for (int u = 0; u < kSetupUnroll; ++u) {
                 const bool ok = (unsigned)jj[u] < (unsigned)K;
@@ -148,6 +153,29 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
         }
         s = warp_sum_u64(s);
         hb = __any_sync(kFull, hb);
+        const int hl = h1 - h0;
+        if (s >= 16ull * hl && s <= kEsc1FlopMax && !hb) {  // at most 64 A entries: jj, lo, hi hold them all
+            int cmin = INT_MAX, cmax = -1;
+            if (sflop) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (hi[u] > lo[u]) {
+                        cmin = min(cmin, __ldg(bcol + lo[u]));
+                        cmax = max(cmax, __ldg(bcol + hi[u] - 1));
+                    }
+                }
+                cmin = __reduce_min_sync(kFull, cmin);
+                cmax = __reduce_max_sync(kFull, cmax);
+            }
+            const int h2 = __shfl_sync(kFull, a2, t);
+            bool next = h2 - h1 == hl && hl <= 32;
+            if (next && lane < hl) next = __ldg(acol + h1 + lane) == jj[0] + 1;
+            next = __all_sync(kFull, next);
+            if (lane == t) {
+                windowed = cmax >= cmin && cmax - cmin < kWinBits;
+                chained = next;
+            }
+        }
         if (lane == t) {
             flop = (long long)s;
             bad = hb;
@@ -235,8 +263,8 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
         if (cls == kClsE1 && f32 >= 16 * lenA) {
             // a column-window row keeps two passes: span of its B rows' first and last
             // columns (B rows are sorted; lenA <= 64 here)
-            int cmin = INT_MAX, cmax = -1;
             if (light) {
+                int cmin = INT_MAX, cmax = -1;
 #pragma unroll
                 for (int u = 0; u < kSetupUnroll; ++u) {
                     if (u < lenA && bl[u] > 0) {
@@ -244,22 +272,17 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
                         cmax = max(cmax, __ldg(bcol + b0[u] + bl[u] - 1));
                     }
                 }
-            } else {
-                for (int p = a0; p < a1; ++p) {
-                    const int j = __ldg(acol + p);
-                    if ((unsigned)j >= (unsigned)K) continue;  // reported above
-                    const int q0 = __ldg(brpt + j), q1 = __ldg(brpt + j + 1);
-                    if (q1 > q0) {
-                        cmin = min(cmin, __ldg(bcol + q0));
-                        cmax = max(cmax, __ldg(bcol + q1 - 1));
-                    }
-                }
+                windowed = cmax >= cmin && cmax - cmin < kWinBits;
             }
-            if (cmax >= cmin && cmax - cmin < kWinBits) staged = 0;
+            if (windowed) staged = 0;
         }
         if (in) sflop[r] = staged;
         if (cls == kClsE1 && staged) atomicAdd(&s_e1one, 1);
     }
+    chained &= cls == kClsE1;
+    if (in) link[r] = chained ? 1 : 0;
+    const int n_chained = __popc(__ballot_sync(kFull, chained));
+    if (lane == 0 && n_chained) atomicAdd(&s_chained, n_chained);
     const unsigned long long wsf = warp_sum_u64((unsigned long long)staged);
     unsigned long long wf = warp_sum_u64((unsigned long long)flop);
     const unsigned wmax = __reduce_max_sync(kFull, (unsigned)f32);
@@ -282,6 +305,7 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
         for (int w = 0; w < kSetupThreads / 32; ++w) ts += s_sflop[w];
         if (ts) atomicAdd(&info->staged_flop, ts);
         if (s_e1one) atomicAdd(&info->e1_one, s_e1one);
+        if (s_chained) atomicAdd(&info->e1_chain, s_chained);
         for (int i = 0; i < 5; ++i)
             if (s_size[i]) atomicAdd(i < 3 ? &info->e1_size[i] : &info->e2_size[i - 3], s_size[i]);
         unsigned long long sn = 0;

@@ -33,6 +33,11 @@ __global__ void k_split_list(const int *__restrict__ list, const int *count_ptr,
     }
 }
 
+// Flags of a row beside the next one (regular.cuh): row r + 1 follows row r; row r belongs
+// to a group of rows of one pattern.
+constexpr unsigned char kLinked = 1;
+constexpr unsigned char kGrouped = 2;
+
 // Numeric re-binning of the E1 rows by their output size (known after the symbolic
 // phase): 0 / 3 = at most 256 / 512 products, fewer than two products per output (a warp /
 // 64 threads per row), 1 = warp hash (at most kSplitNnz outputs: hashing folds the many
@@ -62,8 +67,10 @@ struct PickE1 {
 struct PickStaged {
     const int *soff;
     const int *row_flop;
+    const unsigned char *link;  // rows in groups are dropped (null: there are none)
     __device__ int operator()(int r) const
     {
+        if (link && (link[r] & kGrouped)) return -1;
         if (soff[r + 1] <= soff[r]) return 1;
         return row_flop[r] <= kE1SmallMax ? 0 : (row_flop[r] <= kE1HalfMax ? 3 : 2);
     }

@@ -1,0 +1,482 @@
+// regular.cuh — rows of C on structured grids: consecutive rows whose A entries and whose B
+// rows move on by one column from row to row (stencils and other banded operators) share
+// one pattern, so it is worked out once for a group of rows.  Replaces, for those
+// rows, OpSparse's shared-hash kernels of its middle bins (kernels/symbolic.cuh:74-130,
+// kernels/numeric.cuh:109-205), which hash every product of every row.
+//
+// Row r + 1 follows row r ("link") when A's row r + 1 is A's row r moved by one column and
+// every B row j that A's row r selects is followed by B's row j + 1, its columns moved by one.
+// The product of such rows has the same pattern moved by one, and product number q of each
+// of them goes to the same position.  The relation is checked exactly, entry by entry.
+//
+//   k_setup        A's part of the link, for the rows that fold many products per entry
+//   k_shift_links  B's part: b_link[j]
+//   k_row_links    both: link[r]
+//   k_form_groups  runs of links cut into groups of up to kGroupRows rows; marks their rows
+//   k_group_count  one row counted, all counts written
+//   k_group_rows   numeric: a CTA per group.  The pattern's schedule lists every entry's
+//                  products in ascending j, once.  32 rows at a time, A's and B's values are
+//                  staged in shared memory (a B row once for all rows and A entries that
+//                  reach it) and a lane is a row: a warp walks its share of the schedule with
+//                  one FMA per product of 32 rows and the accumulator in a register.  A
+//                  remainder of at most 16 or 8 rows takes 2 or 4 entries per warp.
+//
+// What bounds it: FP64 issue (a warp's FMA occupies the SM for about 20 cycles; a 78-row
+// run of the 27-point stencil takes 2.5 FMAs per product, 0.80 ms for an 80^3 grid of the
+// 0.93 ms measured); FP32 instruction issue (the compensated sum and three shared loads a
+// product).  The warp hash, which probes and updates shared memory for every product,
+// took 1.91 ms (FP32, 61x47x53 grid: 548 us against 232), the window count of every row
+// 0.58 ms against 0.11 for links, groups and counts.
+#pragma once
+
+#include "lists.cuh"
+
+namespace opsg {
+
+constexpr int kGroupRows = 256;     // rows of a group, at most
+constexpr int kGroupLanes = 32;     // rows computed together: a lane each
+constexpr int kGroupMin = 6;        // shorter runs stay with their class
+constexpr int kGroupAMax = 32;      // A entries of a grouped row: a bit each in an entry's mask
+constexpr int kGroupWindow = 1024;  // rows whose runs one warp cuts
+constexpr int kGroupStage = 9216;   // B values staged for 32 rows, at most
+constexpr int kGroupThreads = 512;
+constexpr int kGroupFlush = 4;      // entries a warp gathers before it writes them
+constexpr int kGroupTop = 1024;     // words of the pattern's trie level 0, at most
+
+// b_link[j] = 1 where row j + 1 is row j moved by one column and all its columns are in
+// [0, cols).  Eight lanes per row.
+static __global__ void __launch_bounds__(256) k_shift_links(const int *__restrict__ rpt, const int *__restrict__ col,
+                                                            int rows, int cols, unsigned char *__restrict__ b_link)
+{
+    const int sub = threadIdx.x & 7;
+    for (long long j = (blockIdx.x * 256ll + threadIdx.x) >> 3; j < rows; j += gridDim.x * 32ll) {
+        bool ok = j + 1 < rows;
+        if (ok) {
+            const int b0 = __ldg(rpt + j), b1 = __ldg(rpt + j + 1), b2 = __ldg(rpt + j + 2);
+            const int n = b1 - b0;
+            ok = b2 - b1 == n && n <= kGroupStage / kGroupLanes;
+            if (ok) {
+                for (int i = sub; i < n; i += 8) {
+                    const int c = __ldg(col + b0 + i), d = __ldg(col + b1 + i);
+                    ok &= d == c + 1 && d < cols && c >= 0;
+                }
+            }
+        }
+        const bool all = __all_sync(255u << (threadIdx.x & 24), ok);
+        if (sub == 0) b_link[j] = all ? 1 : 0;
+    }
+}
+
+// link[r] (in: A's part) and the B part of every B row the row selects, where the row's B
+// values fit the staging area.  Eight lanes per row.
+static __global__ void __launch_bounds__(256) k_row_links(const int *__restrict__ arpt, const int *__restrict__ acol,
+                                                          const int *__restrict__ brpt, int M,
+                                                          const unsigned char *__restrict__ b_link,
+                                                          unsigned char *__restrict__ link)
+{
+    const int sub = threadIdx.x & 7;
+    for (long long r = (blockIdx.x * 256ll + threadIdx.x) >> 3; r < M; r += gridDim.x * 32ll) {
+        bool ok = link[r] & kLinked;
+        int pencils = 0, longest = 0, inner = 0;
+        const unsigned row_lanes = 255u << (threadIdx.x & 24);
+        if (ok) {
+            const int a0 = __ldg(arpt + r), a1 = __ldg(arpt + r + 1);
+            for (int p = a0 + sub; p < a1; p += 8) {
+                const int j = __ldg(acol + p);
+                ok &= __ldg(b_link + j) != 0;
+                longest = max(longest, __ldg(brpt + j + 1) - __ldg(brpt + j));
+                if (p + 1 < a1 && __ldg(acol + p + 1) == j + 1) ++inner;
+                else ++pencils;
+            }
+        }
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1) {
+            pencils += __shfl_xor_sync(row_lanes, pencils, d);
+            inner += __shfl_xor_sync(row_lanes, inner, d);
+            longest = max(longest, __shfl_xor_sync(row_lanes, longest, d));
+        }
+        ok &= (pencils * kGroupLanes + inner) * (longest | 1) + 8 * pencils <= kGroupStage;
+        const bool all = __all_sync(row_lanes, ok);
+        if (sub == 0 && !all) link[r] = 0;
+    }
+}
+
+// Cuts the runs of links into groups (first row, rows) and marks their rows.  A warp takes
+// kGroupWindow rows; runs end at its window.
+static __global__ void __launch_bounds__(128) k_form_groups(int M, unsigned char *__restrict__ link,
+                                                            int2 *__restrict__ groups, DevInfo *info)
+{
+    const int lane = lane_id();
+    const int w0 = ((blockIdx.x * 128 + threadIdx.x) >> 5) * kGroupWindow;
+    if (w0 >= M) return;
+    unsigned mine = 0u;  // lane i: links of rows w0 + 32 i .. + 31
+    for (int i = 0; i < kGroupWindow / 32; ++i) {
+        const int r = w0 + 32 * i + lane;
+        const bool l = r < M && r + 1 < w0 + kGroupWindow && (link[r] & kLinked);
+        const unsigned m = __ballot_sync(kFull, l);
+        if (lane == i) mine = m;
+    }
+    int at = 0;  // rows of the window looked at so far
+    while (at < kGroupWindow) {
+        // next linked row from `at` on
+        unsigned m = mine;
+        const int w = at >> 5;
+        if (lane < w) m = 0u;
+        if (lane == w) m &= kFull << (at & 31);
+        const unsigned any = __ballot_sync(kFull, m != 0u);
+        if (!any) break;
+        const int wl = __ffs(any) - 1;
+        const int s = 32 * wl + __ffs(__shfl_sync(kFull, m, wl)) - 1;
+        // first row from s on without a link: the run's last row
+        m = ~mine;
+        if (lane < (s >> 5)) m = 0u;
+        if (lane == (s >> 5)) m &= kFull << (s & 31);
+        const unsigned any0 = __ballot_sync(kFull, m != 0u);  // never 0: the window's last row has no link
+        const int we = __ffs(any0) - 1;
+        const int e = 32 * we + __ffs(__shfl_sync(kFull, m, we)) - 1;
+        const int len = e - s + 1;
+        const int rest = len % kGroupLanes;
+        const int grouped = len - (rest < kGroupMin ? rest : 0);
+        const int n = (grouped + kGroupRows - 1) / kGroupRows;
+        if (n > 0) {
+            int base = 0;
+            if (lane == 0) base = atomicAdd(&info->groups, n);
+            base = __shfl_sync(kFull, base, 0);
+            if (lane < n) groups[base + lane] = make_int2(w0 + s + kGroupRows * lane, min(kGroupRows, grouped - kGroupRows * lane));
+            for (int i = lane; i < grouped; i += 32) link[w0 + s + i] |= kGrouped;
+        }
+        at = e + 1;
+    }
+}
+
+// Rows of a class list outside the groups: 0 kept, -1 dropped.
+struct PickUngrouped {
+    const unsigned char *link;
+    __device__ int operator()(int r) const { return (link[r] & kGrouped) ? -1 : 0; }
+};
+
+// Counting: the group's first row by column rank, its count for every row.
+static __global__ void __launch_bounds__(RankE1::kThreads, RankE1::kMinBlocks)
+    k_group_count(SpgemmArgs<double> g, const int2 *__restrict__ groups)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const RankSmem<RankE1, double> sm(smem_raw);
+    const int count = g.info->groups;
+    const int levels = rank_levels(g.N, RankE1::kTop);
+    unsigned long long nnz_acc = 0;
+    int n_late = 0;
+    for (int i = blockIdx.x; i < count; i += gridDim.x) {
+        const int2 gr = groups[i];
+        const unsigned long long before = nnz_acc;
+        rank_row<RankE1, false, double>(g, gr.x, sm, levels, nnz_acc, &n_late);  // ends with a barrier
+        if (threadIdx.x == 0) nnz_acc = before + (unsigned long long)gr.y * (nnz_acc - before);
+        const int c = g.c_rpt[gr.x];
+        for (int r = threadIdx.x + 1; r < gr.y; r += RankE1::kThreads) g.c_rpt[gr.x + r] = c;
+    }
+    if (threadIdx.x == 0 && nnz_acc) atomicAdd(&g.info->total_nnz, nnz_acc);
+}
+
+// Copies one value to shared memory without a register.
+template <typename T>
+__device__ __forceinline__ void copy_async(T *dst, const T *src)
+{
+    static_assert(sizeof(T) == 4 || sizeof(T) == 8, "one 4- or 8-byte value");
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"((int)sizeof(T)) : "memory");
+}
+
+// Copies 16 bytes (both addresses aligned to them).
+template <typename T>
+__device__ __forceinline__ void copy_async16(T *dst, const T *src)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+
+template <typename T>
+struct GroupSmem {
+    T b[kGroupStage];                           // B values: slot rows of one pitch
+    T a[kGroupLanes * (kGroupAMax + 1)];        // A values, rows of lenA | 1
+    union {
+        T tile[kGroupThreads / 32][kGroupFlush * (kGroupLanes + 4)];  // a warp's entries by (entry, row)
+        struct {  // while the pattern is worked out
+            unsigned bits[2][kEsc1FlopMax];     // trie levels, then the entries' masks of A entries
+            unsigned pre[2][kEsc1FlopMax];
+        };
+    };
+    unsigned sched[kEsc1FlopMax];      // products by entry: stage offset << 6 | last of its entry << 5 | A entry
+    int col[kEsc1FlopMax];             // the first row's columns
+    unsigned start[kEsc1FlopMax + 4];  // an entry's first product in sched
+    int e_start[kGroupAMax + 1];       // first product of an A entry
+    int e_b0[kGroupAMax];              // its B row's first entry in B
+    int e_len[kGroupAMax];             // and length
+    int e_base[kGroupAMax];            // and its place in b
+    int p_entry[kGroupAMax];           // pencils (runs of entries whose B rows follow one another): first entry
+    int p_entries[kGroupAMax];         // and entries
+    int wsum[32];
+    int next;
+};
+static_assert(2 * (sizeof(GroupSmem<double>) + 1024) <= 227 * 1024 && kGroupTop <= kEsc1FlopMax, "two CTAs an SM");
+
+// The entries of n rows (n <= SW): part threadIdx.x / SW of the schedule by SW lanes, a lane
+// per row, written to C kGroupFlush entries of a row at a time.
+template <int SW, typename T>
+__device__ __forceinline__ void group_fold(GroupSmem<T> &s, int total, int products, int n, int row0, int pa, int pb,
+                                           int *pc, T *pv)
+{
+    using AccT = Acc<T>;
+    constexpr int kParts = kGroupThreads / SW;
+    const int lane = lane_id();
+    const int row = lane % SW;
+    const unsigned lanes = SW == 32 ? kFull : ((1u << (SW & 31)) - 1u) << (lane & ~(SW - 1));
+    const int part = (int)threadIdx.x / SW;
+    // first entry at or after the part's share of the products
+    auto entry_at = [&](int p) {
+        int lo = 0, hi = total;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if ((int)s.start[mid] < p) lo = mid + 1;
+            else hi = mid;
+        }
+        return lo;
+    };
+    const int o0 = entry_at((int)((long long)products * part / kParts));
+    const int o_end = entry_at((int)((long long)products * (part + 1) / kParts));
+    int e = (int)s.start[o0];
+    const int e_end = (int)s.start[o_end];
+    const T *a = s.a + min(row, n - 1) * pa;
+    const T *b = s.b + min(row, n - 1) * pb;
+    T *tile = s.tile[threadIdx.x >> 5] + (lane / SW) * kGroupFlush * (SW + 1);
+    T *put = tile + row;  // this row's next entry
+    // the lane's part of a flush: entry fx of rows fr, fr + SW / kGroupFlush, ...
+    const int fx = row % kGroupFlush, fr = row / kGroupFlush;
+    const int *fcol = s.col + o0 + fx;
+    pc += fr * total + o0 + fx;
+    pv += fr * total + o0 + fx;
+    auto flush = [&]() {
+        __syncwarp(lanes);
+        if (tile + fx * (SW + 1) + row < put) {  // the entry is held (put = tile + held * (SW + 1) + row)
+            const int c = *fcol + row0;
+            const T *from = tile + fx * (SW + 1);
+            int at = 0;
+#pragma unroll
+            for (int r = fr; r < SW; r += SW / kGroupFlush, at += SW / kGroupFlush * total) {
+                if (r < n) {
+                    pc[at] = c + r;
+                    pv[at] = from[r];
+                }
+            }
+        }
+        __syncwarp(lanes);
+        put = tile + row;
+        fcol += kGroupFlush;
+        pc += kGroupFlush;
+        pv += kGroupFlush;
+    };
+    typename AccT::S acc = AccT::zero();
+    auto product = [&](unsigned x, T av, T bv) {
+        acc = AccT::step(acc, av, bv);
+        if (x & 32u) {
+            *put = AccT::fin(acc);
+            acc = AccT::zero();
+            put += SW + 1;
+            if (put == tile + row + kGroupFlush * (SW + 1)) flush();
+        }
+    };
+    for (; e + 4 <= e_end; e += 4) {
+        unsigned x[4];
+        T av[4], bv[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = s.sched[e + u];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            av[u] = a[x[u] & 31u];
+            bv[u] = b[x[u] >> 6];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) product(x[u], av[u], bv[u]);
+    }
+    for (; e < e_end; ++e) {
+        const unsigned x = s.sched[e];
+        product(x, a[x & 31u], b[x >> 6]);
+    }
+    if (put != tile + row) flush();
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kGroupThreads, 2) k_group_rows(SpgemmArgs<T> g, const int2 *__restrict__ groups,
+                                                                 int *cursor)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    GroupSmem<T> &s = *reinterpret_cast<GroupSmem<T> *>(smem_raw);
+    constexpr int NT = kGroupThreads;
+    constexpr int NW = NT / 32;
+    constexpr int PER = kEsc1FlopMax / NT;       // products per thread
+    constexpr int kQuad = 16 / (int)sizeof(T);   // values of a 16-byte copy
+    const int t = threadIdx.x;
+    const int lane = lane_id();
+    const int warp = t >> 5;
+    const int count = g.info->groups;
+    const int levels = rank_levels(g.N, kGroupTop);
+    for (;;) {
+        if (t == 0) s.next = atomicAdd(cursor, 1);
+        __syncthreads();
+        const int it = s.next;
+        if (it >= count) break;
+        const int2 gr = groups[it];
+        const int a0 = __ldg(g.arpt + gr.x);
+        const int len_a = __ldg(g.arpt + gr.x + 1) - a0;
+        const int off = __ldg(g.c_rpt + gr.x);
+        const int pa = len_a | 1;
+        // the pattern's A entries and pencils; every warp works them out, warp 0 stores them
+        int j = -2, b0 = 0, bl = 0;
+        if (lane < len_a) {
+            j = __ldg(g.acol + a0 + lane);
+            b0 = __ldg(g.brpt + j);
+            bl = __ldg(g.brpt + j + 1) - b0;
+        }
+        const int jp = __shfl_up_sync(kFull, j, 1);
+        const bool head = lane < len_a && (lane == 0 || jp != j - 1);
+        const unsigned heads = __ballot_sync(kFull, head);
+        const int pencils = __popc(heads);
+        const int longest = (int)__reduce_max_sync(kFull, (unsigned)bl);
+        // B rows of one odd length: a pencil's rows lie in b as they lie in B, copied 16 bytes
+        // at a time; else every B row gets a row of an odd pitch
+        const bool packed = (longest & 1) && __all_sync(kFull, lane >= len_a || bl == longest);
+        const int pb = longest | 1;
+        const int p = __popc(heads & (lanemask_lt() | (1u << lane))) - 1;  // pencils before and with this entry, less 1
+        int base = (lane + p * (kGroupLanes - 1)) * pb;
+        if (packed) {  // as many values into 16 bytes as the pencil's first value lies in memory
+            const int h = 31 - __clz(heads & (lanemask_lt() | (1u << lane)));  // the pencil's first entry
+            const int first = __shfl_sync(kFull, b0, h);
+            const int want = (int)(((size_t)(g.bval + first) / sizeof(T)) % kQuad);
+            const int k = lane - h;
+            // (8 values a pencil cover the rounding and the shift)
+            base = (base - k * pb + p * 8 + kQuad - 1) / kQuad * kQuad + want + k * pb;
+        }
+        const int p_incl = warp_incl_scan(bl);
+        if (warp == 0) {
+            if (lane < len_a) {
+                s.e_start[lane + 1] = p_incl;
+                s.e_b0[lane] = b0;
+                s.e_len[lane] = bl;
+                s.e_base[lane] = base;
+            }
+            if (head) {
+                const unsigned after = heads & ~(lanemask_lt() | (1u << lane));
+                s.p_entry[p] = lane;
+                s.p_entries[p] = (after ? __ffs(after) - 1 : len_a) - lane;
+            }
+            if (lane == 0) s.e_start[0] = 0;
+        }
+        int words = (int)(((unsigned)g.N - 1u) >> (5 * levels)) + 1;
+        rank_clear<NT>(s.bits[0], words, t);
+        rank_clear<NT>(s.bits[1], kEsc1FlopMax, t);
+        __syncthreads();
+        const int products = min(s.e_start[len_a], kEsc1FlopMax);
+        // A's and B's values of rows [r0, r0 + n) of the group
+        auto stage = [&](int r0, int n) {
+            for (int i = warp; i < n; i += NW)
+                if (lane < len_a)
+                    copy_async(s.a + i * pa + lane, g.aval + a0 + (long long)(r0 + i) * len_a + lane);
+            for (int q = 0; q < pencils; ++q) {
+                const int e = s.p_entry[q], rows = s.p_entries[q] - 1 + n, len = s.e_len[e];
+                const T *src = g.bval + s.e_b0[e] + (long long)r0 * len;
+                T *dst = s.b + s.e_base[e];
+                if (packed) {
+                    const int values = rows * len;
+                    const int lead = min(values, (int)((kQuad - ((size_t)src / sizeof(T)) % kQuad) % kQuad));
+                    const int quads = (values - lead) / kQuad;
+                    for (int i = t; i < quads; i += NT) copy_async16(dst + lead + i * kQuad, src + lead + i * kQuad);
+                    const int rest = values - quads * kQuad;  // before and after the whole quads
+                    if (t < rest) {
+                        const int i = t < lead ? t : t + quads * kQuad;
+                        copy_async(dst + i, src + i);
+                    }
+                } else {
+                    for (int i = warp; i < rows; i += NW)
+                        for (int c = lane; c < len; c += 32) copy_async(dst + i * pb + c, src + i * len + c);
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        stage(0, min(gr.y, kGroupLanes));
+        // the pattern: products' columns, entries and positions
+        unsigned col[PER], idx[PER];
+        int own[PER], at[PER];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const int q = t + k * NT;
+            col[k] = 0u;
+            own[k] = 0;
+            at[k] = 0;
+            if (q < products) {
+                int lo = 0, hi = len_a;
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (s.e_start[mid] <= q) lo = mid;
+                    else hi = mid;
+                }
+                own[k] = lo;
+                const int c = q - s.e_start[lo];
+                at[k] = s.e_base[lo] + c;
+                col[k] = min((unsigned)__ldg(g.bcol + s.e_b0[lo] + c), (unsigned)g.N - 1u);
+            }
+            idx[k] = col[k] >> (5 * levels);
+        }
+        int total = 0;
+        for (int l = 0; l < levels; ++l) {
+            unsigned *bits = s.bits[l & 1], *pre = s.pre[l & 1];
+            const int shift = 5 * (levels - 1 - l);
+#pragma unroll
+            for (int k = 0; k < PER; ++k)
+                if (t + k * NT < products) atomicOr(bits + idx[k], 1u << ((col[k] >> shift) & 31u));
+            __syncthreads();
+            if (l > 0) rank_clear<NT>(s.bits[(l + 1) & 1], kEsc1FlopMax, t);
+            total = rank_prefix<NT>(bits, pre, words, t, warp, lane, s.wsum);
+            words = total;
+#pragma unroll
+            for (int k = 0; k < PER; ++k)
+                if (t + k * NT < products)
+                    idx[k] = pre[idx[k]] + __popc(bits[idx[k]] & ((1u << ((col[k] >> shift) & 31u)) - 1u));
+        }
+        // an entry's products in ascending j: its mask of A entries is one more level
+        unsigned *mask = s.bits[levels & 1];  // zeroed above (levels >= 2) or at the group's start
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            if (t + k * NT < products) {
+                atomicOr(mask + idx[k], 1u << own[k]);
+                s.col[idx[k]] = (int)col[k];
+            }
+        }
+        __syncthreads();
+        rank_prefix<NT>(mask, s.start, total, t, warp, lane, s.wsum);
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            if (t + k * NT < products) {
+                const unsigned m = mask[idx[k]], below = m & ((1u << own[k]) - 1u);
+                const unsigned last = (m >> own[k]) == 1u ? 32u : 0u;
+                s.sched[s.start[idx[k]] + __popc(below)] = ((unsigned)at[k] << 6) | last | (unsigned)own[k];
+            }
+        }
+        if (t == 0) s.start[total] = (unsigned)products;
+        const bool fits = __ldg(g.c_rpt + gr.x + gr.y) - off == gr.y * total;
+        if (t == 0 && !fits) atomicOr(&g.info->flags, kErrCountMismatch);
+        for (int r0 = 0; r0 < gr.y; r0 += kGroupLanes) {
+            const int n = min(kGroupLanes, gr.y - r0);
+            if (r0 > 0) stage(r0, n);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            if (fits) {
+                int *pc = g.c_col + off + r0 * total;
+                T *pv = g.c_val + off + r0 * total;
+                if (n > 16) group_fold<32, T>(s, total, products, n, r0, pa, pb, pc, pv);
+                else if (n > 8) group_fold<16, T>(s, total, products, n, r0, pa, pb, pc, pv);
+                else group_fold<8, T>(s, total, products, n, r0, pa, pb, pc, pv);
+            }
+            __syncthreads();  // the staged values are done with
+        }
+    }
+}
+
+}  // namespace opsg

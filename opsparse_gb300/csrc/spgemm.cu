@@ -24,7 +24,7 @@
 #include <new>
 #include <string>
 
-#include "lists.cuh"
+#include "regular.cuh"
 #include "internal.hpp"
 #include "opsparse_gb300.h"
 
@@ -86,6 +86,7 @@ void set_smem_attrs()
     set_rank_attrs<RankE1, T>();
     set_rank_attrs<RankMid, T>();
     set_rank_attrs<RankLarge, T>();
+    cudaFuncSetAttribute(k_group_rows<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmem<T>));
 }
 
 int ensure_ws(ops_handle_s *h, int M, cudaStream_t st)
@@ -98,7 +99,9 @@ int ensure_ws(ops_handle_s *h, int M, cudaStream_t st)
     const size_t flop_b = align_up(sizeof(int) * (size_t)M, 256);
     const size_t soff_b = align_up(sizeof(int) * ((size_t)M + 1), 256);
     const size_t info_b = align_up(sizeof(DevInfo), 256);
-    const size_t total = lists_b + flop_b + soff_b + info_b + align_up(cub_bytes, 256);
+    const size_t link_b = align_up((size_t)M, 256);
+    const size_t groups_b = align_up(sizeof(int2) * ((size_t)M / kGroupMin + 64), 256);
+    const size_t total = lists_b + flop_b + soff_b + info_b + link_b + groups_b + align_up(cub_bytes, 256);
     if (h->ws) {
         OPS_CUDA(h, cudaFreeAsync(h->ws, st));
         h->ws = nullptr;
@@ -112,7 +115,9 @@ int ensure_ws(ops_handle_s *h, int M, cudaStream_t st)
     h->row_flop = reinterpret_cast<int *>(h->ws + lists_b);
     h->soff = reinterpret_cast<int *>(h->ws + lists_b + flop_b);
     h->info = reinterpret_cast<DevInfo *>(h->ws + lists_b + flop_b + soff_b);
-    h->cub_tmp = h->ws + lists_b + flop_b + soff_b + info_b;
+    h->link = h->ws + lists_b + flop_b + soff_b + info_b;
+    h->groups = reinterpret_cast<int2 *>(h->ws + lists_b + flop_b + soff_b + info_b + link_b);
+    h->cub_tmp = h->ws + lists_b + flop_b + soff_b + info_b + link_b + groups_b;
     h->cub_bytes = cub_bytes;
     h->plan_valid = false;
     return OPS_OK;
@@ -243,7 +248,7 @@ int launch_staged_class(ops_handle_s *h, const GA &gs, int c, const int *list, i
             int *one_large = xl + kXlE1OneLarge * M;
             int *one_half = xl + kXlE1OneHalf * M;
             k_split_list<4, PickStaged><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
-                list, &h->info->counts[c], PickStaged{h->soff, g.row_flop}, one, (int)M, h->info->split1);
+                list, &h->info->counts[c], PickStaged{h->soff, g.row_flop, h->regular ? h->link : nullptr}, one, (int)M, h->info->split1);
             OPS_CUDA(h, cudaGetLastError());
             ++h->launches;
             OPS_CUDA(h, cudaEventRecord(h->ev_x_fork[0], s));
@@ -319,6 +324,37 @@ int launch_staged_class(ops_handle_s *h, const GA &gs, int c, const int *list, i
     return OPS_OK;
 }
 
+// Below this many rows that the next row of A may continue, the groups' four extra launches
+// (about 15 us) are not worth it: a row saves about 4 ns (61x47x53 grid, FP32: 0.27 ms for
+// 150,000 rows), so the sides meet at about 4,000 rows.
+constexpr int kMinChainRows = 4096;
+
+// Groups of rows of one pattern (regular.cuh), where k_setup found enough E1 rows that A's
+// next row repeats: links from B, groups, and the E1 rows outside them (h->regular).
+int form_groups(ops_handle_s *h, const DevInfo &hi, const Mat &A, const Mat &B, cudaStream_t st)
+{
+    h->regular = false;
+    if (hi.e1_chain < kMinChainRows) return OPS_OK;
+    const int M = A.rows, K = A.cols;
+    if (h->b_link_rows < K) {
+        if (h->b_link) OPS_CUDA(h, cudaFreeAsync(h->b_link, st));
+        h->b_link = nullptr;
+        h->b_link_rows = 0;
+        void *p = nullptr;
+        OPS_CUDA(h, cudaMallocFromPoolAsync(&p, (size_t)K, h->pool, st));
+        h->b_link = static_cast<unsigned char *>(p);
+        h->b_link_rows = K;
+    }
+    const int sms = h->num_sms;
+    k_shift_links<<<grid_for(K, 32, sms * 16), 256, 0, st>>>(B.rpt, B.col, K, B.cols, h->b_link);
+    k_row_links<<<grid_for(M, 32, sms * 16), 256, 0, st>>>(A.rpt, A.col, B.rpt, M, h->b_link, h->link);
+    k_form_groups<<<(M + 4 * kGroupWindow - 1) / (4 * kGroupWindow), 128, 0, st>>>(M, h->link, h->groups, h->info);
+    OPS_CUDA(h, cudaGetLastError());
+    h->launches += 3;
+    h->regular = true;
+    return OPS_OK;
+}
+
 // One-pass set-up, once the class sizes are known: when the call has its values, one
 // pass is on and the staged products fit the handle's staging budget, grows the staging
 // area and turns the per-row product counts (k_setup's sflop) into staging offsets.
@@ -367,6 +403,34 @@ int prepare_stage(ops_handle_s *h, const DevInfo &hi, int M, cudaStream_t st)
     h->staged = true;
     h->stage_e1 = hi.e1_one > 0;
     h->stage_e1_all = hi.e1_one == hi.counts[kClsE1];
+    return OPS_OK;
+}
+
+// The groups' counts (symbolic; one row of each is counted) or entries (numeric).
+template <bool kNum, typename T>
+int launch_groups(ops_handle_s *h, const SpgemmArgs<T> &g, int rows, cudaStream_t s)
+{
+    const int most = rows / kGroupMin + 1;
+    if constexpr (kNum) {
+        k_group_rows<T><<<std::min(most, h->num_sms * 2), kGroupThreads, sizeof(GroupSmem<T>), s>>>(
+            g, h->groups, &h->info->next_num.group);
+    } else {
+        SpgemmArgs<double> gc{};
+        gc.arpt = g.arpt;
+        gc.acol = g.acol;
+        gc.brpt = g.brpt;
+        gc.bcol = g.bcol;
+        gc.M = g.M;
+        gc.K = g.K;
+        gc.N = g.N;
+        gc.row_flop = g.row_flop;
+        gc.c_rpt = g.c_rpt;
+        gc.info = g.info;
+        k_group_count<<<std::min(most, h->num_sms * RankE1::kMinBlocks), RankE1::kThreads, RankE1::smem<false>(), s>>>(
+            gc, h->groups);
+    }
+    OPS_CUDA(h, cudaGetLastError());
+    ++h->launches;
     return OPS_OK;
 }
 
@@ -421,6 +485,9 @@ int launch_classes(ops_handle_s *h, const SpgemmArgs<T> &g, cudaStream_t st)
             ++h->launches;
         }
         if (h->timing >= 2) OPS_CUDA(h, cudaEventRecord(h->ev_k[kNum][c][0], s));
+        if (c == kClsE1 && h->regular) {  // the groups of one pattern, then the class's other rows
+            OPS_CHECK((launch_groups<kNum, T>(h, g, n, s)));
+        }
         if (staged && !kNum) {  // one-pass call: numeric into the staging area
             OPS_CHECK(h->op_dtype == OPS_F64 ? launch_staged_class<double>(h, g, c, list, n, s)
                                              : launch_staged_class<float>(h, g, c, list, n, s));
@@ -440,6 +507,16 @@ int launch_classes(ops_handle_s *h, const SpgemmArgs<T> &g, cudaStream_t st)
                 break;
             case kClsE1: {
                 if (!kNum) {  // distinct-column count: one warp per row, table of 2*flop slots
+                    if (h->regular) {
+                        int *two = xl + kXlE1Two * M;
+                        k_split_list<1, PickUngrouped><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
+                            list, &h->info->counts[c], PickUngrouped{h->link}, two, (int)M, &h->info->split1[1]);
+                        k_warp_rows<false, T, 2 * kEsc1FlopMax>
+                            <<<grid_for(n, kWarpRowsThreads / 32, sms * 3), kWarpRowsThreads,
+                               warp_rows_smem<false, T, 2 * kEsc1FlopMax>(), s>>>(g, two, &h->info->split1[1]);
+                        h->launches += 1;
+                        break;
+                    }
                     k_warp_rows<false, T, 2 * kEsc1FlopMax>
                         <<<grid_for(n, kWarpRowsThreads / 32, sms * 3), kWarpRowsThreads,
                            warp_rows_smem<false, T, 2 * kEsc1FlopMax>(), s>>>(g, list, &h->info->counts[c]);
@@ -452,8 +529,9 @@ int launch_classes(ops_handle_s *h, const SpgemmArgs<T> &g, cudaStream_t st)
                 int *half_list = xl + kXlE1Half * M;
                 int *hash_list = xl + kXlE1Hash * M;
                 int *rank_list = xl + kXlE1Rank * M;
-                const int *e1_list = staged ? xl + kXlE1Two * M : list;
-                const int *e1_count = staged ? &h->info->split1[1] : &h->info->counts[c];
+                const bool two = staged || h->regular;
+                const int *e1_list = two ? xl + kXlE1Two * M : list;
+                const int *e1_count = two ? &h->info->split1[1] : &h->info->counts[c];
                 k_split_list<4, PickE1><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
                     e1_list, e1_count, PickE1{g.c_rpt, g.row_flop}, small_list, (int)M, h->info->split);
                 OPS_CUDA(h, cudaGetLastError());
@@ -592,7 +670,7 @@ int run_symbolic(ops_handle_s *h, const Mat &A, const Mat &B, int *c_rpt, long l
     if (M > 0) {
         k_setup<<<(M + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, st>>>(
             A.rpt, A.col, B.rpt, B.col, M, A.cols, B.cols, h->row_flop, h->lists, c_rpt,
-            want_stage ? h->soff : nullptr, h->info, h->th);
+            want_stage ? h->soff : nullptr, h->link, h->info, h->th);
         OPS_CUDA(h, cudaGetLastError());
         ++h->launches;
     }
@@ -614,6 +692,7 @@ int run_symbolic(ops_handle_s *h, const Mat &A, const Mat &B, int *c_rpt, long l
     h->plan_d_flop = (long long)hi.d_flop;
     h->plan_d_len_a = (long long)hi.d_len_a;
     h->staged = false;
+    OPS_CHECK(form_groups(h, hi, A, B, st));
     if (want_stage) OPS_CHECK(prepare_stage(h, hi, M, st));
 
     SpgemmArgs<double> g{};
@@ -803,6 +882,7 @@ int ops_handle_create(ops_handle_t *out)
     if (e == cudaSuccess) {
         set_smem_attrs<double>();
         set_smem_attrs<float>();
+        cudaFuncSetAttribute(k_group_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RankE1::smem<false>());
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
@@ -820,6 +900,7 @@ int ops_handle_destroy(ops_handle_t h)
     cudaDeviceSynchronize();
     for (ops_handle_s *s : h->spare) ops_handle_destroy(s);
     if (h->ws) cudaFree(h->ws);
+    if (h->b_link) cudaFree(h->b_link);
     if (h->dense) cudaFree(h->dense);
     if (h->stage) cudaFree(h->stage);
     for (int c = 0; c < kNumClasses; ++c) {
