@@ -111,7 +111,6 @@ struct DevInfo {
     // zeroed with the rest at the start of the counting phase
     RowCursors next_sym;          // the counting phase's row cursors
     int counts[kNumClasses];      // rows listed in each class
-    int max_flop;                 // clamped to INT_MAX
     unsigned long long total_flop;
     unsigned long long total_nnz;
     int split2[2];                // E2 rows by size, fixed at the symbolic phase: [mid shape, large shape]

@@ -60,11 +60,16 @@ __device__ __forceinline__ void block_add_u64(unsigned long long v, unsigned lon
 // Setup: per-row product count, validation of A's columns, class assignment, and the
 // scatter of row ids into per-class lists (lists[c * M + i]).  One thread per row for
 // rows of at most 8 A entries, whose loads are issued all at once (8 column loads, then
-// 16 row-pointer loads); longer rows are summed cooperatively by their warp, 8 loads in
-// flight per lane.  Rows with no products get nnz 0 immediately and join no list.
+// 16 row-pointer loads); rows of up to kSetupGroupMax entries are summed by eight lanes,
+// longer ones by their warp and the longest by the CTA,
+// 8 loads in flight per lane.  Rows with no products get nnz 0 immediately and join no list.
 // ==================================================================================
-constexpr int kSetupThreads = 512;
+constexpr int kSetupThreads = 256;
 constexpr int kSetupUnroll = 8;
+constexpr int kSetupGroupMax = 128;   // rows of up to this many A entries are summed by eight lanes
+constexpr int kSetupHugeMin = 1024;   // rows of more A entries are summed by the CTA
+constexpr int kSetupHugeRows = 32;    // ... at most this many of a CTA's rows
+constexpr int kSetupGroupUnroll = 4;  // ... which have this many entries each in flight
 
 static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__restrict__ arpt, const int *__restrict__ acol,
                                                         const int *__restrict__ brpt, const int *__restrict__ bcol,
@@ -81,13 +86,25 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
     __shared__ int s_e1one;
     __shared__ int s_size[5];
     __shared__ int s_chained;
+    __shared__ int s_huge_rows;
+    __shared__ int2 s_huge[kSetupHugeRows];  // A entries of the CTA's longest rows
+    __shared__ unsigned long long s_huge_flop[kSetupHugeRows];
+    __shared__ int s_huge_bad[kSetupHugeRows];
+    __shared__ unsigned char s_mid[kSetupThreads / 32][32];       // lanes of the warp's rows of the middle tier
+    __shared__ unsigned char s_mid_flags[kSetupThreads / 32][32]; // 1 bad column, 2 chained, 4 windowed
+    __shared__ unsigned long long s_mid_flop[kSetupThreads / 32][32];
     __shared__ unsigned s_small[kSetupThreads / 32];
     __shared__ int s_flags;
     const int lane = lane_id();
     const int warp = threadIdx.x >> 5;
     if (threadIdx.x < kNumClasses) s_cnt[threadIdx.x] = 0;
+    if (threadIdx.x < kSetupHugeRows) {
+        s_huge_flop[threadIdx.x] = 0ull;
+        s_huge_bad[threadIdx.x] = 0;
+    }
     if (threadIdx.x == 0) {
         s_flags = 0;
+        s_huge_rows = 0;
         s_e1one = 0;
         s_chained = 0;
         for (int i = 0; i < 5; ++i) s_size[i] = 0;
@@ -126,7 +143,124 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
             flop += bl[u];
         }
     }
-    unsigned heavy = __ballot_sync(kFull, in && !light);
+    // rows of 9 to kSetupGroupMax A entries: four at a time by eight lanes each, so that a
+    // warp waits once for four rows' dependent loads (a warp per row waited for each: 27-point
+    // operator of a 57x61x59 grid 63 -> 24 us, of 80^3 188 -> 102 us)
+    const bool mid = in && !light && lenA <= kSetupGroupMax;
+    const unsigned mids = __ballot_sync(kFull, mid);
+    if (mids) {
+        const int sub = lane & 7;
+        if (mid) s_mid[warp][__popc(mids & lanemask_lt())] = (unsigned char)lane;
+        __syncwarp();
+        const int n_mid = __popc(mids);
+        for (int i = 0; i < n_mid; i += 4) {
+            const int k = i + (lane >> 3);
+            const int t = s_mid[warp][min(k, n_mid - 1)];
+            const int h0 = __shfl_sync(kFull, a0, t);
+            const int h1 = __shfl_sync(kFull, a1, t);
+            const int h2 = __shfl_sync(kFull, a2, t);
+            const int hl = h1 - h0;
+            unsigned long long s = 0;
+            bool hb = false;
+            for (int p0 = h0 + sub; p0 < h1; p0 += 8 * kSetupGroupUnroll) {
+                int jj[kSetupGroupUnroll];
+#pragma unroll
+                for (int u = 0; u < kSetupGroupUnroll; ++u) jj[u] = p0 + 8 * u < h1 ? __ldg(acol + p0 + 8 * u) : -1;
+                int lo[kSetupGroupUnroll], hi[kSetupGroupUnroll];
+#pragma unroll
+                for (int u = 0; u < kSetupGroupUnroll; ++u) {
+                    const bool ok = (unsigned)jj[u] < (unsigned)K;
+                    hb |= p0 + 8 * u < h1 && !ok;
+                    lo[u] = ok ? __ldg(brpt + jj[u]) : 0;
+                    hi[u] = ok ? __ldg(brpt + jj[u] + 1) : 0;
+                }
+#pragma unroll
+                for (int u = 0; u < kSetupGroupUnroll; ++u) s += (unsigned long long)(hi[u] - lo[u]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) s += __shfl_xor_sync(kFull, s, d);
+            hb = (__ballot_sync(kFull, hb) >> (lane & 24)) & 255u;
+            // rows that fold many products per entry (at most 64 A entries): do they fall
+            // within a window, and is the next row of A this one moved by one column?
+            const bool many = s >= 16ull * hl && s <= kEsc1FlopMax && !hb;
+            int cmin = INT_MAX, cmax = -1;
+            bool next = many && h2 - h1 == hl && hl <= 32;
+            if (many) {
+                for (int p = h0 + sub; p < h1; p += 8) {
+                    const int j = __ldg(acol + p);
+                    if (next) next = __ldg(acol + h1 + (p - h0)) == j + 1;
+                    if (sflop) {
+                        const int lo = __ldg(brpt + j), hi = __ldg(brpt + j + 1);
+                        if (hi > lo) {
+                            cmin = min(cmin, __ldg(bcol + lo));
+                            cmax = max(cmax, __ldg(bcol + hi - 1));
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+            if (__any_sync(kFull, many)) {
+                next = ((__ballot_sync(kFull, !next) >> (lane & 24)) & 255u) == 0u;
+#pragma unroll
+                for (int d = 1; d < 8; d <<= 1) {
+                    cmin = min(cmin, __shfl_xor_sync(kFull, cmin, d));
+                    cmax = max(cmax, __shfl_xor_sync(kFull, cmax, d));
+                }
+            }
+            if (sub == 0 && k < n_mid) {
+                s_mid_flop[warp][t] = s;
+                s_mid_flags[warp][t] = (unsigned char)((hb ? 1 : 0) | (many && next ? 2 : 0) |
+                                                       (cmax >= cmin && cmax - cmin < kWinBits ? 4 : 0));
+            }
+        }
+        __syncwarp();
+        if (mid) {
+            flop = (long long)s_mid_flop[warp][lane];
+            bad = s_mid_flags[warp][lane] & 1;
+            chained = s_mid_flags[warp][lane] & 2;
+            windowed = s_mid_flags[warp][lane] & 4;
+        }
+    }
+    // the longest rows by the whole CTA: a hub row of 30,000 entries held its warp for 90 us
+    // (kernel 118 -> 66 us on 200,000 nodes with 161 such rows)
+    const bool huge = in && lenA > kSetupHugeMin;
+    int my_huge = -1;
+    if (huge) {
+        my_huge = atomicAdd(&s_huge_rows, 1);
+        if (my_huge < kSetupHugeRows) s_huge[my_huge] = make_int2(a0, a1);
+        else my_huge = -1;  // more of them than the list holds: by their warps
+    }
+    const bool any_huge = __syncthreads_or(huge);
+    for (int h = 0; any_huge && h < min(s_huge_rows, kSetupHugeRows); ++h) {
+        const int2 e = s_huge[h];
+        unsigned long long s = 0;
+        bool hb = false;
+        for (int p0 = e.x; p0 < e.y; p0 += kSetupThreads * kSetupUnroll) {
+            int jj[kSetupUnroll];
+#pragma unroll
+            for (int u = 0; u < kSetupUnroll; ++u) {
+                const int p = p0 + u * kSetupThreads + (int)threadIdx.x;
+                jj[u] = p < e.y ? __ldg(acol + p) : 0;
+                hb |= (unsigned)jj[u] >= (unsigned)K;
+                if (p >= e.y) jj[u] = -1;
+            }
+#pragma unroll
+            for (int u = 0; u < kSetupUnroll; ++u) {
+                if ((unsigned)jj[u] < (unsigned)K)
+                    s += (unsigned long long)(__ldg(brpt + jj[u] + 1) - __ldg(brpt + jj[u]));
+            }
+        }
+        s = warp_sum_u64(s);
+        if (lane == 0 && s) atomicAdd(&s_huge_flop[h], s);
+        if (hb) s_huge_bad[h] = 1;
+    }
+    if (any_huge) __syncthreads();
+    if (my_huge >= 0) {
+        flop = (long long)s_huge_flop[my_huge];
+        bad = s_huge_bad[my_huge] != 0;
+    }
+    unsigned heavy = __ballot_sync(kFull, in && !light && !mid && my_huge < 0);
     while (heavy) {
         const int t = __ffs(heavy) - 1;
         heavy &= heavy - 1u;
@@ -134,13 +268,14 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
         const int h1 = __shfl_sync(kFull, a1, t);
         unsigned long long s = 0;
         bool hb = false;
-        int jj[kSetupUnroll], lo[kSetupUnroll], hi[kSetupUnroll];
         for (int p0 = h0; p0 < h1; p0 += 32 * kSetupUnroll) {
+            int jj[kSetupUnroll];
 #pragma unroll
             for (int u = 0; u < kSetupUnroll; ++u) {
                 const int p = p0 + u * 32 + lane;
                 jj[u] = p < h1 ? __ldg(acol + p) : -1;
             }
+            int lo[kSetupUnroll], hi[kSetupUnroll];
 #pragma unroll
             for (int u = 0; u < kSetupUnroll; ++u) {
                 const bool ok = (unsigned)jj[u] < (unsigned)K;
@@ -153,29 +288,6 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
         }
         s = warp_sum_u64(s);
         hb = __any_sync(kFull, hb);
-        const int hl = h1 - h0;
-        if (s >= 16ull * hl && s <= kEsc1FlopMax && !hb) {  // at most 64 A entries: jj, lo, hi hold them all
-            int cmin = INT_MAX, cmax = -1;
-            if (sflop) {
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    if (hi[u] > lo[u]) {
-                        cmin = min(cmin, __ldg(bcol + lo[u]));
-                        cmax = max(cmax, __ldg(bcol + hi[u] - 1));
-                    }
-                }
-                cmin = __reduce_min_sync(kFull, cmin);
-                cmax = __reduce_max_sync(kFull, cmax);
-            }
-            const int h2 = __shfl_sync(kFull, a2, t);
-            bool next = h2 - h1 == hl && hl <= 32;
-            if (next && lane < hl) next = __ldg(acol + h1 + lane) == jj[0] + 1;
-            next = __all_sync(kFull, next);
-            if (lane == t) {
-                windowed = cmax >= cmin && cmax - cmin < kWinBits;
-                chained = next;
-            }
-        }
         if (lane == t) {
             flop = (long long)s;
             bad = hb;
@@ -285,7 +397,6 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
     if (lane == 0 && n_chained) atomicAdd(&s_chained, n_chained);
     const unsigned long long wsf = warp_sum_u64((unsigned long long)staged);
     unsigned long long wf = warp_sum_u64((unsigned long long)flop);
-    const unsigned wmax = __reduce_max_sync(kFull, (unsigned)f32);
     const unsigned wsmall = __reduce_add_sync(kFull, small_nnz);
     if (lane == 0) {
         s_flop[warp] = wf;
@@ -313,7 +424,6 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
         if (sn) atomicAdd(&info->total_nnz, sn);
         if (s_flags) atomicOr(&info->flags, s_flags);
     }
-    if (lane == 0 && wmax) atomicMax(&info->max_flop, (int)wmax);
     __syncthreads();
     if (cls > kClsR8) lists[(size_t)cls * M + s_base[cls] + my_off] = r;
 }
