@@ -153,6 +153,19 @@ int ops_spgemm(ops_handle_t handle, int dtype, int32_t rows_a, int32_t cols_a, i
                const int32_t *b_rpt, const int32_t *b_col, const void *b_val, int64_t b_nnz,
                int32_t **c_rpt, int32_t **c_col, void **c_val, int64_t *c_nnz, void *stream);
 
+/* ops_spgemm in two halves, for callers that allocate C themselves once its size is known: the
+ * same work (one pass where the handle's mode and the inputs allow it) and the same results.
+ * ops_spgemm_begin fills the caller's c_rpt and returns nnz(C); ops_spgemm_finish, the next
+ * call on the handle, fills c_col and c_val (nnz(C) each) on the same stream for the same
+ * matrices.  Both synchronize the stream.  finish without a begin, or after another
+ * multiplication on the handle, returns OPS_NOT_SUPPORTED.  The matrices' arrays must stay
+ * as they are between the two.  No OpSparse counterpart. */
+int ops_spgemm_begin(ops_handle_t handle, int dtype, int32_t rows_a, int32_t cols_a, int32_t cols_b,
+                     const int32_t *a_rpt, const int32_t *a_col, const void *a_val, int64_t a_nnz,
+                     const int32_t *b_rpt, const int32_t *b_col, const void *b_val, int64_t b_nnz,
+                     int32_t *c_rpt, int64_t *c_nnz, void *stream);
+int ops_spgemm_finish(ops_handle_t handle, int32_t *c_col, void *c_val, void *stream);
+
 /* Symbolic phase: fills the caller's c_rpt (rows_a + 1 int32, device) with C's row
  * pointers and returns nnz(C) in *c_nnz.  Keeps the row classification on the handle
  * for a following ops_spgemm_numeric on the same A and B.  Synchronizes the stream. */
@@ -228,6 +241,9 @@ int ops_batch_check(ops_batch_t batch, void *stream);
 /* Device pointers of C_b (views into the batch's storage, valid until destroy). */
 int ops_batch_result(ops_batch_t batch, int32_t index, int32_t **c_rpt, int32_t **c_col, void **c_val,
                      int64_t *c_nnz);
+/* The same for every problem at once: c_rpt, c_col, c_val and c_nnz are host arrays of one
+ * element per problem. */
+int ops_batch_results(ops_batch_t batch, int32_t **c_rpt, int32_t **c_col, void **c_val, int64_t *c_nnz);
 int ops_batch_info(ops_batch_t batch, int32_t *segments, int64_t *flop, int64_t *nnz);
 /* How the batch was planned: *persistent = 1 when one setup kernel and one persistent kernel
  * per row-size queue and phase cover all its problems (ops_tuning.batch_persistent), with

@@ -190,10 +190,27 @@ class Handle:
         c_col, c_val = self.numeric(A, B, c_rpt, nnz, stream=stream)
         return CsrMatrix(A.rows, B.cols, c_rpt, c_col, c_val)
 
-    # -- one-shot (library-allocated outputs) ----------------------------------
+    # -- one call (one pass where the handle's mode allows it) -------------------
     def spgemm_oneshot(self, A: CsrMatrix, B: CsrMatrix, stream=None) -> CsrMatrix:
-        """C = A * B through ops_spgemm; the library's arrays are copied into torch and freed."""
+        """C = A * B in one pass where the handle's mode and the inputs allow it.  The library
+        fills torch tensors; on a stream other than the current one it allocates C itself, and
+        its arrays are copied into tensors of the current stream and freed."""
         torch = _torch()
+        if stream is None or stream == torch.cuda.current_stream():
+            nnz = C.c_int64(0)
+            a = A.ptrs()
+            b = B.ptrs()
+            st = _stream_ptr(stream)
+            dev = A.rpt.device
+            c_rpt = torch.empty(A.rows + 1, dtype=torch.int32, device=dev)
+            check(self.lib.ops_spgemm_begin(self.h, _dtype_code(A.val), A.rows, A.cols, B.cols, a[0], a[1], a[2], A.nnz,
+                                            b[0], b[1], b[2], B.nnz, c_rpt.data_ptr(), C.byref(nnz), st), self.h)
+            n = int(nnz.value)
+            c_col = torch.empty(n, dtype=torch.int32, device=dev)
+            c_val = torch.empty(n, dtype=A.val.dtype, device=dev)
+            check(self.lib.ops_spgemm_finish(self.h, c_col.data_ptr() if n else None, c_val.data_ptr() if n else None,
+                                             st), self.h)
+            return CsrMatrix(A.rows, B.cols, c_rpt, c_col, c_val)
         rp, cp, vp = C.c_void_p(), C.c_void_p(), C.c_void_p()
         nnz = C.c_int64(0)
         a = A.ptrs()
@@ -246,6 +263,7 @@ class Batch:
                                         C.byref(out), C.c_void_p(self.stream.cuda_stream)), handle.h)
         self.b = out
         self.n = n
+        self._found = None
 
     def execute(self, use_graph: bool = True):
         check(self.lib.ops_batch_execute(self.b, 1 if use_graph else 0, C.c_void_p(self.stream.cuda_stream)),
@@ -281,27 +299,57 @@ class Batch:
                               device="cuda").cpu().numpy()
         return rpt, col, val
 
+    def _results(self):
+        """Every problem's place in the batch's arrays: (base tensors, offsets, counts), the
+        arrays of problems that lie one behind the other wrapped as one tensor."""
+        if self._found is None:
+            torch = _torch()
+            n = self.n
+            rp, cp, vp, nnz = ((kind * max(n, 1))() for kind in (C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64))
+            check(self.lib.ops_batch_results(self.b, rp, cp, vp, nnz), self.h.h)
+            vsize, vstr = (8, "<f8") if self.dtype == torch.float64 else (4, "<f4")
+            dev = self.pairs[0][0].rpt.device if n else "cuda"
+
+            def wrap(ptrs, counts, size, typestr):
+                views, start = [None] * n, 0
+                while start < n:
+                    end, at = start, ptrs[start]
+                    while end < n and ptrs[end] == at:
+                        at += counts[end] * size
+                        end += 1
+                    total = sum(counts[start:end])
+                    base = torch.as_tensor(_DevArray(ptrs[start], total, typestr), device=dev) if total else None
+                    at = 0
+                    for i in range(start, end):
+                        views[i] = (base, at)
+                        at += counts[i]
+                    start = end
+                return views
+
+            rows = [A.rows + 1 for A, _ in self.pairs]
+            self._found = (wrap(rp, rows, 4, "<i4"), wrap(cp, list(nnz), 4, "<i4"), wrap(vp, list(nnz), vsize, vstr),
+                           rows, list(nnz))
+        return self._found
+
     def result_device(self, i: int):
         """(rpt, col, val, nnz) of C_i as torch views of the batch's device storage (valid
         until close())."""
         torch = _torch()
-        rp, cp, vp, nnz = C.c_void_p(), C.c_void_p(), C.c_void_p(), C.c_int64(0)
-        check(self.lib.ops_batch_result(self.b, i, C.byref(rp), C.byref(cp), C.byref(vp), C.byref(nnz)), self.h.h)
-        A = self.pairs[i][0]
-        n = int(nnz.value)
-        dev = A.rpt.device
-        vstr = "<f8" if self.dtype == torch.float64 else "<f4"
-        rpt = torch.as_tensor(_DevArray(rp.value, A.rows + 1, "<i4"), device=dev)
+        rpt, col, val, rows, nnz = self._results()
+        base, at = rpt[i]
+        r = base[at:at + rows[i]]
+        n = nnz[i]
         if n == 0:
-            return rpt, torch.empty(0, dtype=torch.int32, device=dev), torch.empty(0, dtype=self.dtype, device=dev), 0
-        col = torch.as_tensor(_DevArray(cp.value, n, "<i4"), device=dev)
-        val = torch.as_tensor(_DevArray(vp.value, n, vstr), device=dev)
-        return rpt, col, val, n
+            dev = base.device
+            return r, torch.empty(0, dtype=torch.int32, device=dev), torch.empty(0, dtype=self.dtype, device=dev), 0
+        (cb, ca), (vb, va) = col[i], val[i]
+        return r, cb[ca:ca + n], vb[va:va + n], n
 
     def close(self):
         if getattr(self, "b", None):
             self.lib.ops_batch_destroy(self.b)
             self.b = None
+            self._found = None
 
     def __del__(self):
         try:

@@ -102,6 +102,8 @@ _SIGS = {
     "ops_spgemm_check": (C.c_int, [P, P]),
     "ops_flop": (C.c_int, [I32, I32, P, P, P, P, C.POINTER(I64), P]),
     "ops_flop_noalloc": (C.c_int, [I32, I32, P, P, P, P, C.POINTER(I64), P]),
+    "ops_spgemm_begin": (C.c_int, [P, C.c_int, I32, I32, I32, P, P, P, I64, P, P, P, I64, P, C.POINTER(I64), P]),
+    "ops_spgemm_finish": (C.c_int, [P, P, P, P]),
     "ops_free": (C.c_int, [P, P]),
     "ops_spgemm_backward": (C.c_int, [P, C.c_int, I32, I32, I32, P, P, P, I64, P, P, P, I64, P, P, P, P, P, P]),
     "ops_handle_set_map_budget": (C.c_int, [P, C.c_size_t]),
@@ -109,6 +111,7 @@ _SIGS = {
     "ops_batch_create": (C.c_int, [P, C.c_int, I32, C.POINTER(BatchItem), C.POINTER(P), P]),
     "ops_batch_execute": (C.c_int, [P, C.c_int, P]),
     "ops_batch_check": (C.c_int, [P, P]),
+    "ops_batch_results": (C.c_int, [P, C.POINTER(P), C.POINTER(P), C.POINTER(P), C.POINTER(I64)]),
     "ops_batch_result": (C.c_int, [P, I32, C.POINTER(P), C.POINTER(P), C.POINTER(P), C.POINTER(I64)]),
     "ops_batch_info": (C.c_int, [P, C.POINTER(I32), C.POINTER(I64), C.POINTER(I64)]),
     "ops_batch_queues": (C.c_int, [P, C.POINTER(I32), C.POINTER(I64), C.POINTER(I64)]),

@@ -183,13 +183,15 @@ __global__ void k_batch_last(int *a_last, int a_nnz, int *b_last, int b_nnz)
 
 int flat_grid(long long total, int sms) { return (int)std::max<long long>(1, std::min<long long>((total + kFlatChunk - 1) / kFlatChunk, (long long)sms * 16)); }
 
-// Per-problem row_ptr rebased to start at 0, written to the result arena.
+// Per-problem row_ptr rebased to start at 0, written to the result arena, and each problem's
+// first and last entry in its segment's C.
 __global__ void k_batch_rebase(const Item *__restrict__ items, int first, int count, const int *__restrict__ c_rpt,
-                               int *out)
+                               int *out, int2 *__restrict__ extent)
 {
     for (int b = blockIdx.x; b < count; b += gridDim.x) {
         const Item it = items[first + b];
         const int base = c_rpt[it.row_base];
+        if (threadIdx.x == 0) extent[first + b] = make_int2(base, c_rpt[it.row_base + it.rows]);
         for (int r = threadIdx.x; r <= it.rows; r += blockDim.x) out[it.c_rpt_base + r] = c_rpt[it.row_base + r] - base;
     }
 }
@@ -202,6 +204,8 @@ struct ops_batch_s {
     int n = 0;
     std::vector<Item> items;     // host copy
     Item *d_items = nullptr;
+    int2 *d_extent = nullptr;    // each problem's entries in its segment's C (behind d_items)
+    std::vector<int2> extent;    // host copy
     std::vector<Segment> segs;
     int *c_rpt_arena = nullptr;  // all rebased per-problem row pointers
     void *mem = nullptr;         // one allocation for every segment's inputs and row pointers
@@ -287,7 +291,7 @@ int alloc_segment_c(ops_batch_s *b, ops_handle_s *h, Segment &s, size_t vs, cuda
     s.c_val = cv;
     if (s.count > 0) {
         k_batch_rebase<<<std::min(s.count, 65535), 256, 0, st>>>(b->d_items, s.first, s.count, s.c_rpt,
-                                                                b->c_rpt_arena);
+                                                                b->c_rpt_arena, b->d_extent);
         OPS_CUDA(h, cudaGetLastError());
     }
     return OPS_OK;
@@ -597,9 +601,11 @@ extern "C" int ops_batch_create(ops_handle_t h, int dtype, int32_t count, const 
     }
     {
         void *p = nullptr;
-        cudaError_t e = cudaMallocFromPoolAsync(&p, sizeof(Item) * std::max(count, 1), h->pool, st);
+        const size_t items_b = align_up(sizeof(Item) * (size_t)std::max(count, 1), 256);
+        cudaError_t e = cudaMallocFromPoolAsync(&p, items_b + sizeof(int2) * (size_t)std::max(count, 1), h->pool, st);
         if (e != cudaSuccess) return bail(fail(h, status_of(e), "allocating batch descriptors"));
         b->d_items = static_cast<Item *>(p);
+        b->d_extent = reinterpret_cast<int2 *>(static_cast<unsigned char *>(p) + items_b);
         void *f = nullptr;
         e = cudaMallocFromPoolAsync(&f, sizeof(unsigned long long) * std::max(count, 1), h->pool, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_items, b->items.data(), sizeof(Item) * count, cudaMemcpyHostToDevice, st);
@@ -711,7 +717,11 @@ extern "C" int ops_batch_create(ops_handle_t h, int dtype, int32_t count, const 
     bool persistent = false;
     OPS_CHECK_B(plan_persistent(b, h, vs, st, persistent));
     if (!persistent) OPS_CHECK_B(plan_segments(b, h, vs, st));
-    cudaError_t e = cudaStreamSynchronize(st);
+    b->extent.resize(count);
+    cudaError_t e = cudaSuccess;
+    if (count > 0)
+        e = cudaMemcpyAsync(b->extent.data(), b->d_extent, sizeof(int2) * count, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return bail(fail(h, status_of(e), "batch create"));
     *out = b;
     return OPS_OK;
@@ -833,23 +843,40 @@ extern "C" int ops_batch_check(ops_batch_t b, void *stream)
     return OPS_OK;
 }
 
+namespace {
+
+void batch_result_of(const ops_batch_s *b, const Segment &seg, int index, int32_t **c_rpt, int32_t **c_col,
+                     void **c_val, int64_t *c_nnz)
+{
+    const int2 x = b->extent[index];
+    const size_t vs = b->dtype == OPS_F64 ? 8 : 4;
+    *c_rpt = b->c_rpt_arena + b->items[index].c_rpt_base;
+    *c_col = seg.c_col + x.x;
+    *c_val = static_cast<unsigned char *>(seg.c_val) + vs * (size_t)x.x;
+    *c_nnz = x.y - x.x;
+}
+
+}  // namespace
+
 extern "C" int ops_batch_result(ops_batch_t b, int32_t index, int32_t **c_rpt, int32_t **c_col, void **c_val,
                                 int64_t *c_nnz)
 {
     if (!b || index < 0 || index >= b->n || !c_rpt || !c_col || !c_val || !c_nnz) return OPS_INVALID_ARGUMENT;
-    const Item &it = b->items[index];
-    const Segment *seg = nullptr;
+    for (const Segment &s : b->segs) {
+        if (index >= s.first && index < s.first + s.count) {
+            batch_result_of(b, s, index, c_rpt, c_col, c_val, c_nnz);
+            return OPS_OK;
+        }
+    }
+    return OPS_INVALID_ARGUMENT;
+}
+
+extern "C" int ops_batch_results(ops_batch_t b, int32_t **c_rpt, int32_t **c_col, void **c_val, int64_t *c_nnz)
+{
+    if (!b || (b->n > 0 && (!c_rpt || !c_col || !c_val || !c_nnz))) return OPS_INVALID_ARGUMENT;
     for (const Segment &s : b->segs)
-        if (index >= s.first && index < s.first + s.count) seg = &s;
-    if (!seg) return OPS_INVALID_ARGUMENT;
-    int base = 0, end = 0;
-    OPS_CUDA(b->owner, cudaMemcpy(&base, seg->c_rpt + it.row_base, sizeof(int), cudaMemcpyDeviceToHost));
-    OPS_CUDA(b->owner, cudaMemcpy(&end, seg->c_rpt + it.row_base + it.rows, sizeof(int), cudaMemcpyDeviceToHost));
-    const size_t vs = b->dtype == OPS_F64 ? 8 : 4;
-    *c_rpt = b->c_rpt_arena + it.c_rpt_base;
-    *c_col = seg->c_col + base;
-    *c_val = static_cast<unsigned char *>(seg->c_val) + vs * (size_t)base;
-    *c_nnz = end - base;
+        for (int i = s.first; i < s.first + s.count; ++i)
+            batch_result_of(b, s, i, c_rpt + i, c_col + i, c_val + i, c_nnz + i);
     return OPS_OK;
 }
 

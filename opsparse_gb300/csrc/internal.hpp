@@ -84,6 +84,10 @@ struct ops_handle_s {
     // into C after the scan
     int one_pass = 1;              // 0 off, 1 on above kMinStageFlop staged products, 2 on
     int op_dtype = -1;             // value type of the call in progress, -1 = two passes
+    bool begun = false;            // ops_spgemm_begin has run, ops_spgemm_finish has not
+    int begun_dtype = -1;
+    int *begun_rpt = nullptr;      // its c_rpt
+    const void *begun_aval = nullptr, *begun_bval = nullptr;
     const void *op_aval = nullptr, *op_bval = nullptr;
     bool staged = false;           // the counting phase of the call in progress stages
     bool stage_e1 = false;         // ... and some of its rows are E1 rows

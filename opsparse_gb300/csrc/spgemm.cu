@@ -657,6 +657,8 @@ int run_symbolic(ops_handle_s *h, const Mat &A, const Mat &B, int *c_rpt, long l
     const int M = A.rows;
     OPS_CHECK(ensure_ws(h, std::max(M, 1), st));
     h->plan_valid = false;
+    h->begun = false;
+    h->staged = false;
     h->launches = 0;
     std::memset(h->kmeasured, 0, sizeof(h->kmeasured));
     if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[0], st));
@@ -1074,6 +1076,8 @@ int ops_spgemm_numeric(ops_handle_t h, int dtype, int32_t rows_a, int32_t cols_a
         const Mat B{cols_a, cols_b, b_rpt, b_col, b_val};
         if (h->plan_nnz > 0 && (!c_col || !c_val || !a_val || !b_val))
             return fail(h, OPS_INVALID_ARGUMENT, "null values or output");
+        h->begun = false;
+        h->staged = false;  // rows that a begun call staged
         if (dtype == OPS_F64)
             return run_numeric<double>(h, A, B, c_rpt, c_col, static_cast<double *>(c_val), st);
         return run_numeric<float>(h, A, B, c_rpt, c_col, static_cast<float *>(c_val), st);
@@ -1175,6 +1179,72 @@ int ops_spgemm(ops_handle_t h, int dtype, int32_t rows_a, int32_t cols_a, int32_
         return OPS_OK;
     } catch (...) {
         return fail(h, OPS_EXCEPTION, "exception in ops_spgemm");
+    }
+}
+
+int ops_spgemm_begin(ops_handle_t h, int dtype, int32_t rows_a, int32_t cols_a, int32_t cols_b,
+                     const int32_t *a_rpt, const int32_t *a_col, const void *a_val, int64_t a_nnz,
+                     const int32_t *b_rpt, const int32_t *b_col, const void *b_val, int64_t b_nnz, int32_t *c_rpt,
+                     int64_t *c_nnz, void *stream)
+{
+    if (!h || !c_rpt || !c_nnz) return fail(h, OPS_INVALID_ARGUMENT, "null handle or output");
+    if (dtype_size(dtype) == 0) return fail(h, OPS_INVALID_ARGUMENT, "unknown dtype");
+    try {
+        h->last_error.clear();
+        h->begun = false;
+        OPS_CHECK(check_mat_args(h, rows_a, cols_a, a_rpt, a_col, a_nnz));
+        OPS_CHECK(check_mat_args(h, cols_a, cols_b, b_rpt, b_col, b_nnz));
+        if ((a_nnz > 0 && !a_val) || (b_nnz > 0 && !b_val)) return fail(h, OPS_INVALID_ARGUMENT, "null values");
+        const Mat A{rows_a, cols_a, a_rpt, a_col, a_val};
+        const Mat B{cols_a, cols_b, b_rpt, b_col, b_val};
+        long long nnz = 0;
+        h->op_dtype = dtype;
+        h->op_aval = a_val;
+        h->op_bval = b_val;
+        const int s = run_symbolic(h, A, B, c_rpt, &nnz, static_cast<cudaStream_t>(stream));
+        h->op_dtype = -1;
+        h->op_aval = h->op_bval = nullptr;
+        if (s != OPS_OK) {
+            h->staged = false;
+            return s;
+        }
+        h->begun = true;
+        h->begun_dtype = dtype;
+        h->begun_rpt = c_rpt;
+        h->begun_aval = a_val;
+        h->begun_bval = b_val;
+        *c_nnz = nnz;
+        return OPS_OK;
+    } catch (...) {
+        return fail(h, OPS_EXCEPTION, "exception in ops_spgemm_begin");
+    }
+}
+
+int ops_spgemm_finish(ops_handle_t h, int32_t *c_col, void *c_val, void *stream)
+{
+    if (!h) return OPS_INVALID_ARGUMENT;
+    if (!h->begun || !h->plan_valid) return fail(h, OPS_NOT_SUPPORTED, "ops_spgemm_finish without ops_spgemm_begin");
+    h->begun = false;
+    try {
+        h->last_error.clear();
+        struct StagedScope {  // staged rows belong to this call alone
+            ops_handle_s *h;
+            ~StagedScope() { h->staged = false; }
+        } staged_scope{h};
+        if (h->plan_nnz > 0 && (!c_col || !c_val)) return fail(h, OPS_INVALID_ARGUMENT, "null output");
+        cudaStream_t st = static_cast<cudaStream_t>(stream);
+        const Mat A{h->plan_M, h->plan_K, h->plan_arpt, h->plan_acol, h->begun_aval};
+        const Mat B{h->plan_K, h->plan_N, h->plan_brpt, h->plan_bcol, h->begun_bval};
+        if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[5], st));
+        OPS_CHECK(h->begun_dtype == OPS_F64
+                      ? run_numeric<double>(h, A, B, h->begun_rpt, c_col, static_cast<double *>(c_val), st)
+                      : run_numeric<float>(h, A, B, h->begun_rpt, c_col, static_cast<float *>(c_val), st));
+        if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[6], st));
+        OPS_CHECK(check_flags(h, st));
+        fill_timings(h, true);
+        return OPS_OK;
+    } catch (...) {
+        return fail(h, OPS_EXCEPTION, "exception in ops_spgemm_finish");
     }
 }
 
