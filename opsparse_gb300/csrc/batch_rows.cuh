@@ -5,10 +5,11 @@
 // setup kernel walks the rows of every segment of every problem and pushes each row into one
 // of five global queues by its product count:
 //   kQ128:  at most 128 products;
-//   kQ256:  129 .. min(256, warp_max) products;
-//   kQ512:  257 .. warp_max (<= 512) products;
-//   kQE1:   warp_max+1 .. 1,024 products (and at most 1,024 A entries);
-//   kQMid:  1,025 .. 4,096 products (and at most 1,280 A entries).
+//   kQ256:  at most min(256, warp_max) products (and at most 128 A entries);
+//   kQ512:  at most warp_max (<= 512) products (and at most 192 A entries);
+//   kQE1:   at most 1,024 products (and at most 512 A entries);
+//   kQMid:  at most 4,096 products (and at most 1,280 A entries).
+// A row joins the first that takes it.
 // Rows beyond all five are only counted; a batch that has any runs the per-segment pipeline
 // instead.  Each queue is then drained by ONE persistent kernel per phase that spans every
 // problem: its warps (or CTAs) take rows through the queue's atomic cursor until it is
@@ -93,7 +94,8 @@ static __global__ void __launch_bounds__(256) k_batch_setup(const SpgemmArgs<dou
             const_cast<int *>(g.row_flop)[r] = flop > INT_MAX ? INT_MAX : (int)flop;
             if (flop == 0) g.c_rpt[r] = 0;
             else if (flop <= kBatchQ128) cls = kQ128;
-            else if (flop <= warp_max) cls = flop <= kBatchQ256 ? kQ256 : kQ512;
+            else if (flop <= warp_max && flop <= kBatchQ256 && lenA <= RankS::kAEntries) cls = kQ256;
+            else if (flop <= warp_max && lenA <= RankM::kAEntries) cls = kQ512;
             else if (flop <= RankE1::kCap && lenA <= RankE1::kAEntries) cls = kQE1;
             else if (flop <= RankMid::kCap && lenA <= RankMid::kAEntries) cls = kQMid;
             else cls = kQBeyond;

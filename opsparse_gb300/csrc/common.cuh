@@ -20,7 +20,7 @@ enum RowClass : int {
     kClsR16 = 1,  // flop <= 16, lenA <= 16 : 16 lanes per row
     kClsR32 = 2,  // flop <= 32, lenA <= 32 : one warp per row
     kClsW = 3,    // flop <= 128            : one warp per row, column rank
-    kClsE1 = 4,   // flop <= 1024, lenA <= 1024   : column rank (64 or 128 threads) or warp hash
+    kClsE1 = 4,   // flop <= 1024, lenA <= 512   : column rank (64 or 128 threads) or warp hash
     kClsE2 = 5,   // flop <= 13312, lenA <= 2560  : column rank (512 or 1,024 threads)
     kClsD = 6,    // larger                 : whole-GPU stable radix sort (dense accumulator fallback)
     kNumClasses = 7
@@ -48,7 +48,7 @@ constexpr int kNumLists = kNumClasses + kNumExtraLists;
 constexpr int kSmallFlopMax = 8;   // R8 rows: symbolic inside k_setup, numeric k_small_rows
 constexpr int kWarpFlopMax = 128;  // W rows: a warp ranks at most 128 products
 constexpr int kEsc1FlopMax = 1024;
-constexpr int kEsc1AMax = 1024;
+constexpr int kEsc1AMax = 512;
 constexpr int kEsc2FlopMax = 13312;
 constexpr int kEsc2AMax = 2560;
 // Entries of more than kBlockFoldMin products fold in kFoldBlocks consecutive blocks of
@@ -89,13 +89,21 @@ enum : int {
 
 // Row sizes of the shapes that compute the E1 and E2 rows (rank.cuh).
 constexpr int kE1SmallMax = 256;
+constexpr int kE1SmallAMax = 128;
 constexpr int kE1HalfMax = 512;
+constexpr int kE1HalfAMax = 192;
+
+// Shape of an E1 row: 0, 1, 2 = at most kE1SmallMax, kE1HalfMax, kEsc1FlopMax products.
+__host__ __device__ constexpr int e1_shape(int flop, int len_a)
+{
+    return flop <= kE1SmallMax && len_a <= kE1SmallAMax ? 0 : (flop <= kE1HalfMax && len_a <= kE1HalfAMax ? 1 : 2);
+}
 constexpr int kE2MidMax = 4096;
 constexpr int kE2MidAMax = 1280;
 
 // Row cursors of one phase's kernels (a CTA draws its next row from its kernel's cursor).
 struct RowCursors {
-    int e1_half;   // E1 rows of the 512-product shape
+    int e1_half;   // E1 rows of the 512-product shape (kE1Half)
     int e1;        // E1 rows of the 1,024-product shape
     int mid;       // E2 rows of the mid shape
     int large;     // E2 rows of the large shape
@@ -117,7 +125,7 @@ struct DevInfo {
     int split1[4];                // E1 rows of a one-pass call (PickStaged)
     unsigned long long staged_flop;  // products of the rows a one-pass call may stage
     int e1_one;                   // E1 rows a one-pass call may stage
-    int e1_size[3];               // E1 rows of at most 256, 512 and 1,024 products
+    int e1_size[3];               // E1 rows by shape (e1_shape)
     int e2_size[2];               // E2 rows of the mid and the large shape
     int e1_chain;                 // E1 rows whose A row the next row of A repeats, moved by one column
     int groups;                   // groups of rows of one pattern (regular.cuh)

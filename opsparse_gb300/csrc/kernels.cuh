@@ -342,7 +342,7 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
             cls = kClsW;
         } else if (flop <= th.e1 && lenA <= kEsc1AMax) {
             cls = kClsE1;
-            atomicAdd(&s_size[flop <= kE1SmallMax ? 0 : (flop <= kE1HalfMax ? 1 : 2)], 1);
+            atomicAdd(&s_size[e1_shape(f32, lenA)], 1);
         } else if (flop <= th.e2 && lenA <= kEsc2AMax) {
             cls = kClsE2;
             atomicAdd(&s_size[flop <= kE2MidMax && lenA <= kE2MidAMax ? 3 : 4], 1);

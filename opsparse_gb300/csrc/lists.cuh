@@ -39,40 +39,47 @@ constexpr unsigned char kLinked = 1;
 constexpr unsigned char kGrouped = 2;
 
 // Numeric re-binning of the E1 rows by their output size (known after the symbolic
-// phase): 0 / 3 = at most 256 / 512 products, fewer than two products per output (a warp /
-// 64 threads per row), 1 = warp hash (at most kSplitNnz outputs: hashing folds the many
-// products per output cheaply), 2 = the others (128 threads per row).
+// phase): 0 / 3 = the rank shapes of a warp / 64 threads (fewer than two products per
+// output), 1 = warp hash (at most kSplitNnz outputs: hashing folds the many products per
+// output cheaply), 2 = the 128-thread rank shape.
 constexpr int kSplitNnz = 256;
 static_assert(RankW::kCap >= kWarpFlopMax && RankE1::kCap >= kEsc1FlopMax && RankE1::kAEntries >= kEsc1AMax &&
                   RankLarge::kCap >= kEsc2FlopMax && RankLarge::kAEntries >= kEsc2AMax,
               "every class's rows fit its shapes");
-static_assert(RankS::kCap >= kE1SmallMax && RankM::kCap >= kE1HalfMax && RankMid::kCap >= kE2MidMax &&
-                  RankMid::kAEntries >= kE2MidAMax,
+static_assert(RankS::kCap >= kE1SmallMax && RankS::kAEntries >= kE1SmallAMax && RankM::kCap >= kE1HalfMax &&
+                  RankM::kAEntries >= kE1HalfAMax && RankMid::kCap >= kE2MidMax && RankMid::kAEntries >= kE2MidAMax,
               "every size's rows fit its shape");
+static_assert(2 * (kSplitNnz + 1) > kE1HalfMax, "rows of list 2 have the E1 shape");
 
 struct PickE1 {
     const int *c_rpt;
     const int *row_flop;
+    const int *arpt;
     __device__ int operator()(int r) const
     {
         const int nnz = c_rpt[r + 1] - c_rpt[r];
         const int f = row_flop[r];
-        if (f <= kE1HalfMax && f < 2 * nnz) return f <= kE1SmallMax ? 0 : 3;
+        if (f <= kE1HalfMax && f < 2 * nnz) {
+            const int shape = e1_shape(f, arpt[r + 1] - arpt[r]);
+            return shape == 0 ? 0 : (shape == 1 ? 3 : 2);
+        }
         return nnz <= kSplitNnz ? 1 : 2;
     }
 };
 
 // E1 rows of a one-pass call: 1 = not staged, else (a staging slot of one or more products)
-// 0, 3, 2 = at most 256, 512, 1,024 products.
+// 0, 3, 2 = the rank shape of a warp, 64 threads, 128 threads.
 struct PickStaged {
     const int *soff;
     const int *row_flop;
+    const int *arpt;
     const unsigned char *link;  // rows in groups are dropped (null: there are none)
     __device__ int operator()(int r) const
     {
         if (link && (link[r] & kGrouped)) return -1;
         if (soff[r + 1] <= soff[r]) return 1;
-        return row_flop[r] <= kE1SmallMax ? 0 : (row_flop[r] <= kE1HalfMax ? 3 : 2);
+        const int shape = e1_shape(row_flop[r], arpt[r + 1] - arpt[r]);
+        return shape == 0 ? 0 : (shape == 1 ? 3 : 2);
     }
 };
 

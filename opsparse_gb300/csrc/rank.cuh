@@ -43,8 +43,9 @@ namespace opsg {
 // NT threads compute a row of at most NT * PER products (product q = tid + k * NT is a
 // thread's k-th), GROUPS rows at a time per CTA (GROUPS > 1: warps).  ACAP bounds the A
 // entries with a non-empty B row, MINB the CTAs per SM the registers must allow, TOP the
-// words of level 0.
-template <int NT, int PER, int ACAP, int GROUPS, int MINB, int TOP>
+// words of level 0.  RELOAD64: 64-bit values of B are loaded when they are folded, not held
+// in registers from the expansion on.
+template <int NT, int PER, int ACAP, int GROUPS, int MINB, int TOP, bool RELOAD64 = false>
 struct RankShape {
     static_assert(NT % 32 == 0 && (GROUPS == 1 || NT == 32), "rows of several warps take a whole CTA");
     static constexpr int kGroup = NT;
@@ -59,6 +60,11 @@ struct RankShape {
     // the widest shape writes entries of unrepeated columns straight to C (its shared memory
     // holds values of repeated columns only) and reloads its operands
     static constexpr bool kWide = kCap > 4096;
+    template <typename T>
+    static constexpr bool reload()
+    {
+        return kWide || (RELOAD64 && sizeof(T) == 8);
+    }
     static constexpr int kLevel0 = !kWide && kCap > TOP ? kCap : TOP;
     static_assert(kCap % 128 == 0 && TOP % 4 == 0 && kCap < 65536 && ACAP < 4096, "packed scan, 16-bit product numbers");
 
@@ -91,11 +97,16 @@ struct RankShape {
     }
 };
 
-// Rows of at most 128, 256, 512, 1,024, 4,096 and 13,312 products.
-using RankW = RankShape<32, 4, 128, 8, 4, 256>;
-using RankS = RankShape<32, 8, 256, 4, 7, 256>;
-using RankM = RankShape<64, 8, 512, 1, 13, 512>;
-using RankE1 = RankShape<128, 8, 1024, 1, 6, 1024>;
+// Rows of at most 128, 256, 512, 1,024, 4,096 and 13,312 products.  The kernels are bound by
+// latency at 40-60% of the warps an SM holds, so the A entries of the shapes in between are
+// few enough (128, 192 and 512; longer rows take the next shape) for their shared memory and
+// registers to let 36, 34 and 32 warps run: rows of 352 products 54.6 -> 49.3 us for 10,000
+// (FP64), of 176 products 48.8 -> 45.0 us for 20,000, of 64 products 36.5 -> 33.8 us for
+// 30,000, against 28, 26, 24 and 32 warps.
+using RankW = RankShape<32, 4, 128, 4, 10, 256>;
+using RankS = RankShape<32, 8, 128, 4, 9, 256, true>;
+using RankM = RankShape<64, 8, 192, 1, 17, 512, true>;
+using RankE1 = RankShape<128, 8, 512, 1, 8, 1024>;
 using RankMid = RankShape<512, 8, 1280, 1, 2, 2048>;
 using RankLarge = RankShape<1024, 13, 2560, 1, 1, 1024>;
 
@@ -292,6 +303,7 @@ __device__ __forceinline__ void rank_row(const SpgemmArgs<T> &g, int r, const Ra
     constexpr int NT = Sh::kGroup;
     constexpr int PER = Sh::kPer;
     constexpr int NW = Sh::kWarps;
+    constexpr bool kReload = Sh::template reload<T>();
     const int lane = lane_id();
     const int t = NT == 32 ? lane : (int)threadIdx.x;
     const int warp = NT == 32 ? 0 : t >> 5;
@@ -311,8 +323,8 @@ __device__ __forceinline__ void rank_row(const SpgemmArgs<T> &g, int r, const Ra
     rank_clear<NT>(sm.bits(0), words, t);
     if (levels > 1) rank_clear<NT>(sm.bits(1), row_products, t);
     if constexpr (kNum) {
-        if (t < Sh::kCap / 32) sm.multi()[t] = 0u;
         static_assert(Sh::kCap / 32 <= NT, "a word per thread");
+        if (t < Sh::kCap / 32) sm.multi()[t] = 0u;
     }
     if (t == 0) sm.late()[0] = 0;
 
@@ -380,7 +392,7 @@ __device__ __forceinline__ void rank_row(const SpgemmArgs<T> &g, int r, const Ra
                 if (c + lane < n) {
                     const int kb = sm.off()[own[k]] + c + lane;
                     col[k] = (unsigned)__ldg(g.bcol + kb);
-                    if constexpr (kNum && !Sh::kWide) bv[k] = __ldg(g.bval + kb);
+                    if constexpr (kNum && !kReload) bv[k] = __ldg(g.bval + kb);
                 }
             }
         }
@@ -448,6 +460,10 @@ __device__ __forceinline__ void rank_row(const SpgemmArgs<T> &g, int r, const Ra
         }
         group_sync<NT>();
     } else {
+        auto b_value = [&](int k) -> T {
+            if constexpr (kReload) return __ldg(g.bval + sm.off()[own[k]] + t + k * NT);
+            else return bv[k];
+        };
         // positions
         {
             unsigned *up = sm.bits(levels - 1);
@@ -470,7 +486,7 @@ __device__ __forceinline__ void rank_row(const SpgemmArgs<T> &g, int r, const Ra
                     if (k * NT >= n) break;
                     const bool in = t + k * NT < n;
                     if (in && !((late >> k) & 1u) && (int)idx[k] < n_expect) pc[idx[k]] = (int)col[k];
-                    rank_fold_lanes<T>(in, idx[k], s, in ? sm.a_value(g, own[k]) : T(0), bv[k]);
+                    rank_fold_lanes<T>(in, idx[k], s, in ? sm.a_value(g, own[k]) : T(0), in ? b_value(k) : T(0));
                 }
                 if (lane < min(total, n_expect)) g.c_val[off + lane] = AccT::fin(s);
                 if (lane == 0) {
@@ -516,10 +532,7 @@ __device__ __forceinline__ void rank_row(const SpgemmArgs<T> &g, int r, const Ra
             if (t + k * NT < n && !((late >> k) & 1u)) {  // one product of each column
                 const bool direct = !((listed >> k) & 1u);
                 S s = AccT::zero();
-                if (direct) {
-                    const T b = Sh::kWide ? __ldg(g.bval + sm.off()[own[k]] + t + k * NT) : bv[k];
-                    s = AccT::step(s, sm.a_value(g, own[k]), b);
-                }
+                if (direct) s = AccT::step(s, sm.a_value(g, own[k]), b_value(k));
                 if constexpr (Sh::kWide) {
                     if ((int)idx[k] < n_expect) {
                         g.c_col[off + (int)idx[k]] = (int)col[k];
@@ -539,7 +552,8 @@ __device__ __forceinline__ void rank_row(const SpgemmArgs<T> &g, int r, const Ra
                 for (int k = 0; k < PER; ++k) {
                     if (k * NT >= n) break;
                     const bool in = (listed >> k) & 1u;
-                    rank_fold_entries<T>(in, own[k], val + idx[k], in ? sm.a_value(g, own[k]) : T(0), bv[k]);
+                    rank_fold_entries<T>(in, own[k], val + idx[k], in ? sm.a_value(g, own[k]) : T(0),
+                                         in ? b_value(k) : T(0));
                 }
             }
         } else if (n_late > 0) {

@@ -248,7 +248,7 @@ int launch_staged_class(ops_handle_s *h, const GA &gs, int c, const int *list, i
             int *one_large = xl + kXlE1OneLarge * M;
             int *one_half = xl + kXlE1OneHalf * M;
             k_split_list<4, PickStaged><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
-                list, &h->info->counts[c], PickStaged{h->soff, g.row_flop, h->regular ? h->link : nullptr}, one, (int)M, h->info->split1);
+                list, &h->info->counts[c], PickStaged{h->soff, g.row_flop, g.arpt, h->regular ? h->link : nullptr}, one, (int)M, h->info->split1);
             OPS_CUDA(h, cudaGetLastError());
             ++h->launches;
             OPS_CUDA(h, cudaEventRecord(h->ev_x_fork[0], s));
@@ -533,7 +533,7 @@ int launch_classes(ops_handle_s *h, const SpgemmArgs<T> &g, cudaStream_t st)
                 const int *e1_list = two ? xl + kXlE1Two * M : list;
                 const int *e1_count = two ? &h->info->split1[1] : &h->info->counts[c];
                 k_split_list<4, PickE1><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
-                    e1_list, e1_count, PickE1{g.c_rpt, g.row_flop}, small_list, (int)M, h->info->split);
+                    e1_list, e1_count, PickE1{g.c_rpt, g.row_flop, g.arpt}, small_list, (int)M, h->info->split);
                 OPS_CUDA(h, cudaGetLastError());
                 ++h->launches;
                 cudaStream_t sx = fork_x(0, s);
