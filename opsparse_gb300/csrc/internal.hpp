@@ -105,6 +105,7 @@ struct ops_handle_s {
     const int *plan_arpt = nullptr, *plan_acol = nullptr, *plan_brpt = nullptr, *plan_bcol = nullptr;
     int counts[kNumClasses] = {};
     int e1_size[3] = {}, e2_size[2] = {};  // E1 and E2 rows by shape (DevInfo)
+    bool small = false;           // one kernel takes every row (k_rank_all)
     bool regular = false;         // some E1 rows are in groups of one pattern (regular.cuh)
     long long plan_flop = 0;
     long long plan_nnz = 0;

@@ -113,6 +113,10 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
 
     const int r = blockIdx.x * kSetupThreads + threadIdx.x;
     const bool in = r < M;
+    if (r == M - 1) {  // the ends of the arrays that are scanned
+        c_rownnz[M] = 0;
+        if (sflop) sflop[M] = 0;
+    }
     int a0 = 0, a1 = 0, a2 = 0;
     if (in) {
         a0 = arpt[r];
@@ -426,6 +430,34 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
     }
     __syncthreads();
     if (cls > kClsR8) lists[(size_t)cls * M + s_base[cls] + my_off] = r;
+}
+
+// Exclusive scan in place of x[0, n) by one CTA: for row counts of small problems, where the
+// two launches of a device-wide scan cost more than its bandwidth.
+constexpr int kScanMax = 32769;
+
+static __global__ void __launch_bounds__(1024) k_scan_rows(int *__restrict__ x, int n)
+{
+    __shared__ int s_sums[32];
+    int carry = 0;
+    for (int i0 = 0; i0 < n; i0 += 4096) {
+        const int i = i0 + 4 * (int)threadIdx.x;
+        int v[4], sum = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            v[u] = i + u < n ? x[i + u] : 0;
+            sum += v[u];
+        }
+        int total = 0;
+        int run = carry + block_inclusive_scan(sum, s_sums, &total) - sum;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (i + u < n) x[i + u] = run;
+            run += v[u];
+        }
+        carry += total;
+        __syncthreads();  // s_sums is used again
+    }
 }
 
 // ==================================================================================

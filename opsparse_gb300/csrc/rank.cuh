@@ -722,4 +722,33 @@ __global__ void __launch_bounds__(Sh::kThreads, Sh::kMinBlocks)
     }
 }
 
+// Small problems, every row of at most RankS::kCap products (E1 rows of at most
+// RankS::kAEntries A entries) by one kernel, a warp per row in row order: the classes' kernels,
+// each a launch and two events on a stream of its own, take longer to launch than to run.
+// Symbolic: the rows that k_setup left to count (not those of at most r8 products and A
+// entries).  Does nothing where k_setup found a bad column of A.
+template <bool kNum, typename T>
+__global__ void __launch_bounds__(RankS::kThreads, RankS::kMinBlocks) k_rank_all(SpgemmArgs<T> g, int r8)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (!kNum && g.info->flags) return;
+    const int warp = threadIdx.x >> 5;
+    const RankSmem<RankS, T> sm(smem_raw + (size_t)warp * RankS::template group_bytes<kNum>());
+    const int levels = rank_levels(g.N, RankS::kTop);
+    unsigned long long nnz_acc = 0;
+    int n_late = 0;
+    const int nwarps = gridDim.x * RankS::kGroups;
+    for (int r = blockIdx.x * RankS::kGroups + warp; r < g.M; r += nwarps) {
+        const int f = __ldg(g.row_flop + r);
+        if (f == 0 || f > RankS::kCap) continue;
+        const int len_a = __ldg(g.arpt + r + 1) - __ldg(g.arpt + r);
+        if (!kNum && f <= r8 && len_a <= r8) continue;
+        if (f > RankS::kAEntries && len_a > RankS::kAEntries) continue;
+        rank_row<RankS, kNum, T>(g, r, sm, levels, nnz_acc, &n_late);
+    }
+    if constexpr (!kNum) {
+        if (lane_id() == 0 && nnz_acc) atomicAdd(&g.info->total_nnz, nnz_acc);
+    }
+}
+
 }  // namespace opsg

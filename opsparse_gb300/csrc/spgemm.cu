@@ -41,6 +41,7 @@ struct Mat {
     int rows, cols;
     const int *rpt, *col;
     const void *val;
+    long long nnz = -1;  // -1: not known
 };
 
 template <typename Sh, typename T>
@@ -86,6 +87,8 @@ void set_smem_attrs()
     set_rank_attrs<RankE1, T>();
     set_rank_attrs<RankMid, T>();
     set_rank_attrs<RankLarge, T>();
+    cudaFuncSetAttribute(k_rank_all<true, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RankS::smem<true>());
+    cudaFuncSetAttribute(k_rank_all<false, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RankS::smem<false>());
     cudaFuncSetAttribute(k_group_rows<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmem<T>));
 }
 
@@ -182,6 +185,20 @@ int grid_for(long long work_items, int per_block, int cap)
 {
     long long b = (work_items + per_block - 1) / per_block;
     return (int)std::max<long long>(1, std::min<long long>(b, cap));
+}
+
+// Row pointers of C (or staging offsets) from counts, in place: x[0, M] -> exclusive prefix.
+int scan_rows(ops_handle_s *h, int *x, int M, cudaStream_t st)
+{
+    if (M + 1 <= kScanMax) {
+        k_scan_rows<<<1, 1024, 0, st>>>(x, M + 1);
+        OPS_CUDA(h, cudaGetLastError());
+    } else {
+        size_t cb = h->cub_bytes;
+        OPS_CUDA(h, cub::DeviceScan::ExclusiveSum(h->cub_tmp, cb, x, x, M + 1, st));
+    }
+    ++h->launches;
+    return OPS_OK;
 }
 
 // Classes whose rows a one-pass call computes in the counting phase: all but R8 (counted
@@ -397,9 +414,7 @@ int prepare_stage(ops_handle_s *h, const DevInfo &hi, int M, cudaStream_t st)
             ++h->launches;
         }
     }
-    size_t cb = h->cub_bytes;
-    OPS_CUDA(h, cub::DeviceScan::ExclusiveSum(h->cub_tmp, cb, h->soff, h->soff, M + 1, st));
-    ++h->launches;
+    OPS_CHECK(scan_rows(h, h->soff, M, st));
     h->staged = true;
     h->stage_e1 = hi.e1_one > 0;
     h->stage_e1_all = hi.e1_one == hi.counts[kClsE1];
@@ -644,6 +659,27 @@ int count_status(ops_handle_s *h, const DevInfo &d)
     return OPS_OK;
 }
 
+// Whether a problem is launched as a small one: few rows, short ones on average.
+constexpr int kSmallRows = 16384;
+constexpr double kSmallMeanProducts = 96;
+
+bool small_problem(const ops_handle_s *h, const Mat &A, const Mat &B)
+{
+    if (A.rows == 0 || A.rows > kSmallRows || A.nnz < 0 || B.nnz < 0 || h->timing >= 2) return false;
+    if (h->op_dtype >= 0 && h->one_pass == 2) return false;  // staged at any size
+    return (double)A.nnz * (double)B.nnz <= kSmallMeanProducts * (double)A.rows * (double)A.cols;
+}
+
+template <bool kNum, typename T>
+int launch_all(ops_handle_s *h, const SpgemmArgs<T> &g, cudaStream_t st)
+{
+    const int ctas = std::min((g.M + RankS::kGroups - 1) / RankS::kGroups, h->num_sms * RankS::kMinBlocks);
+    k_rank_all<kNum, T><<<ctas, RankS::kThreads, RankS::smem<kNum>(), st>>>(g, h->th.r8);
+    OPS_CUDA(h, cudaGetLastError());
+    ++h->launches;
+    return OPS_OK;
+}
+
 // Counting phase: class sizes (one host sync), the classes' kernels, the row_ptr scan and
 // nnz(C) (a second sync).  early_alloc (ops_spgemm): where C at one entry per product fits
 // kEarlyAllocBytes and no row is a D row, the second sync is left out; *c_nnz is then -1,
@@ -662,25 +698,55 @@ int run_symbolic(ops_handle_s *h, const Mat &A, const Mat &B, int *c_rpt, long l
     h->launches = 0;
     std::memset(h->kmeasured, 0, sizeof(h->kmeasured));
     if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[0], st));
-    OPS_CUDA(h, cudaMemsetAsync(h->info, 0, sizeof(DevInfo), st));
-    OPS_CUDA(h, cudaMemsetAsync(c_rpt + M, 0, sizeof(int), st));
     // a one-pass call also gets the per-row products it may stage (made into offsets once
     // the staging area is known to fit)
     const bool want_stage = h->one_pass != 0 && h->op_dtype >= 0;
-    if (want_stage) OPS_CUDA(h, cudaMemsetAsync(h->soff + M, 0, sizeof(int), st));
-    if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[1], st));
-    if (M > 0) {
-        k_setup<<<(M + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, st>>>(
-            A.rpt, A.col, B.rpt, B.col, M, A.cols, B.cols, h->row_flop, h->lists, c_rpt,
-            want_stage ? h->soff : nullptr, h->link, h->info, h->th);
-        OPS_CUDA(h, cudaGetLastError());
-        ++h->launches;
+    SpgemmArgs<double> g{};
+    g.arpt = A.rpt;
+    g.acol = A.col;
+    g.brpt = B.rpt;
+    g.bcol = B.col;
+    g.M = M;
+    g.K = A.cols;
+    g.N = B.cols;
+    g.row_flop = h->row_flop;
+    g.c_rpt = c_rpt;
+    g.info = h->info;
+    // small problems: every row by one kernel, the scan behind it, one host sync for all of
+    // it.  It is launched before the row sizes are known, where their mean is small; if some
+    // row is too large for it, the usual pipeline starts over.
+    bool small = small_problem(h, A, B);
+    DevInfo hi;
+    for (;;) {
+        OPS_CUDA(h, cudaMemsetAsync(h->info, 0, sizeof(DevInfo), st));
+        if (M == 0) OPS_CUDA(h, cudaMemsetAsync(c_rpt, 0, sizeof(int), st));
+        if (M == 0 && want_stage) OPS_CUDA(h, cudaMemsetAsync(h->soff, 0, sizeof(int), st));
+        if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[1], st));
+        if (M > 0) {
+            k_setup<<<(M + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, st>>>(
+                A.rpt, A.col, B.rpt, B.col, M, A.cols, B.cols, h->row_flop, h->lists, c_rpt,
+                want_stage ? h->soff : nullptr, h->link, h->info, h->th);
+            OPS_CUDA(h, cudaGetLastError());
+            ++h->launches;
+        }
+        if (small) {
+            if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[2], st));
+            OPS_CHECK((launch_all<false, double>(h, g, st)));
+            if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[3], st));
+            OPS_CHECK(scan_rows(h, c_rpt, M, st));
+            if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[4], st));
+        }
+        OPS_CUDA(h, cudaMemcpyAsync(h->h_info, h->info, sizeof(DevInfo), cudaMemcpyDeviceToHost, st));
+        if (h->timing && !small) OPS_CUDA(h, cudaEventRecord(h->ev_t[2], st));
+        OPS_CUDA(h, cudaStreamSynchronize(st));
+        hi = *h->h_info;
+        if (!small || (hi.counts[kClsE2] == 0 && hi.counts[kClsD] == 0 && hi.e1_size[1] == 0 && hi.e1_size[2] == 0))
+            break;
+        small = false;
     }
-    OPS_CUDA(h, cudaMemcpyAsync(h->h_info, h->info, sizeof(DevInfo), cudaMemcpyDeviceToHost, st));
-    if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[2], st));
-    OPS_CUDA(h, cudaStreamSynchronize(st));
-    const DevInfo hi = *h->h_info;
-    if (hi.flags & kErrBadColumn) return fail(h, OPS_INVALID_CSR, "A has a column index outside [0, cols)");
+    if (hi.flags & kErrBadColumn)
+        return fail(h, OPS_INVALID_CSR, small ? "A or B has a column index outside [0, cols)"
+                                              : "A has a column index outside [0, cols)");
     if (hi.flags & kErrRowFlopOverflow)
         return fail(h, OPS_INT32_OVERFLOW, "a row of C has more than INT32_MAX intermediate products");
     std::memcpy(h->counts, hi.counts, sizeof(h->counts));
@@ -694,24 +760,24 @@ int run_symbolic(ops_handle_s *h, const Mat &A, const Mat &B, int *c_rpt, long l
     h->plan_d_flop = (long long)hi.d_flop;
     h->plan_d_len_a = (long long)hi.d_len_a;
     h->staged = false;
+    h->small = small;
+    h->regular = false;
+    h->plan_arpt = A.rpt;
+    h->plan_acol = A.col;
+    h->plan_brpt = B.rpt;
+    h->plan_bcol = B.col;
+    if (small) {
+        OPS_CHECK(count_status(h, hi));
+        *c_nnz = (long long)hi.total_nnz;
+        h->plan_nnz = (long long)hi.total_nnz;
+        h->plan_valid = true;
+        return OPS_OK;
+    }
     OPS_CHECK(form_groups(h, hi, A, B, st));
     if (want_stage) OPS_CHECK(prepare_stage(h, hi, M, st));
-
-    SpgemmArgs<double> g{};
-    g.arpt = A.rpt;
-    g.acol = A.col;
-    g.brpt = B.rpt;
-    g.bcol = B.col;
-    g.M = M;
-    g.K = A.cols;
-    g.N = B.cols;
-    g.row_flop = h->row_flop;
-    g.c_rpt = c_rpt;
-    g.info = h->info;
     OPS_CHECK((launch_classes<false, double>(h, g, st)));
     if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[3], st));
-    size_t cb = h->cub_bytes;
-    OPS_CUDA(h, cub::DeviceScan::ExclusiveSum(h->cub_tmp, cb, c_rpt, c_rpt, M + 1, st));
+    OPS_CHECK(scan_rows(h, c_rpt, M, st));
     if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[4], st));
     const int vs = h->op_dtype >= 0 ? dtype_size(h->op_dtype) : 0;
     if (early_alloc && vs > 0 && hi.counts[kClsD] == 0 &&
@@ -727,10 +793,6 @@ int run_symbolic(ops_handle_s *h, const Mat &A, const Mat &B, int *c_rpt, long l
         *c_nnz = (long long)h2.total_nnz;
         h->plan_nnz = (long long)h2.total_nnz;
     }
-    h->plan_arpt = A.rpt;
-    h->plan_acol = A.col;
-    h->plan_brpt = B.rpt;
-    h->plan_bcol = B.col;
     h->plan_valid = true;
     return OPS_OK;
 }
@@ -758,6 +820,7 @@ int run_numeric(ops_handle_s *h, const Mat &A, const Mat &B, const int *c_rpt, i
     g.c_val = c_val;
     g.info = h->info;
     g.hash_slots = h->hash_slots;
+    if (h->small) return launch_all<true, T>(h, g, st);
     return launch_classes<true, T>(h, g, st);
 }
 
@@ -1028,7 +1091,7 @@ int ops_handle_subclass_rows(ops_handle_t h, int32_t *out, int n)
         DevInfo d{};
         OPS_CUDA(h, cudaMemcpy(&d, h->info, sizeof(DevInfo), cudaMemcpyDeviceToHost));
         // a one-pass call computes its staged E1 rows while counting (split1)
-        v[0] = d.split[0] + d.split[3] + d.split1[0] + d.split1[3];
+        v[0] = d.split[0] + d.split[3] + d.split1[0] + d.split1[3] + (h->small ? h->e1_size[0] : 0);
         v[1] = d.split[1];
         v[2] = d.split[2] + d.split1[2];
         v[3] = d.split2[0];
@@ -1049,8 +1112,8 @@ int ops_spgemm_symbolic(ops_handle_t h, int32_t rows_a, int32_t cols_a, int32_t 
         OPS_CHECK(check_mat_args(h, rows_a, cols_a, a_rpt, a_col, a_nnz));
         OPS_CHECK(check_mat_args(h, cols_a, cols_b, b_rpt, b_col, b_nnz));
         cudaStream_t st = static_cast<cudaStream_t>(stream);
-        const Mat A{rows_a, cols_a, a_rpt, a_col, nullptr};
-        const Mat B{cols_a, cols_b, b_rpt, b_col, nullptr};
+        const Mat A{rows_a, cols_a, a_rpt, a_col, nullptr, a_nnz};
+        const Mat B{cols_a, cols_b, b_rpt, b_col, nullptr, b_nnz};
         h->op_dtype = -1;  // no values: two passes
         long long nnz = 0;
         OPS_CHECK(run_symbolic(h, A, B, c_rpt, &nnz, st));
@@ -1110,8 +1173,8 @@ int ops_spgemm(ops_handle_t h, int dtype, int32_t rows_a, int32_t cols_a, int32_
         OPS_CHECK(check_mat_args(h, cols_a, cols_b, b_rpt, b_col, b_nnz));
         if ((a_nnz > 0 && !a_val) || (b_nnz > 0 && !b_val)) return fail(h, OPS_INVALID_ARGUMENT, "null values");
         cudaStream_t st = static_cast<cudaStream_t>(stream);
-        const Mat A{rows_a, cols_a, a_rpt, a_col, a_val};
-        const Mat B{cols_a, cols_b, b_rpt, b_col, b_val};
+        const Mat A{rows_a, cols_a, a_rpt, a_col, a_val, a_nnz};
+        const Mat B{cols_a, cols_b, b_rpt, b_col, b_val, b_nnz};
         // the values are known before the counting phase: the R16, R32 and W rows may run
         // their numeric kernels there (one pass); reset whichever way the call returns
         struct OnePassScope {
@@ -1195,8 +1258,8 @@ int ops_spgemm_begin(ops_handle_t h, int dtype, int32_t rows_a, int32_t cols_a, 
         OPS_CHECK(check_mat_args(h, rows_a, cols_a, a_rpt, a_col, a_nnz));
         OPS_CHECK(check_mat_args(h, cols_a, cols_b, b_rpt, b_col, b_nnz));
         if ((a_nnz > 0 && !a_val) || (b_nnz > 0 && !b_val)) return fail(h, OPS_INVALID_ARGUMENT, "null values");
-        const Mat A{rows_a, cols_a, a_rpt, a_col, a_val};
-        const Mat B{cols_a, cols_b, b_rpt, b_col, b_val};
+        const Mat A{rows_a, cols_a, a_rpt, a_col, a_val, a_nnz};
+        const Mat B{cols_a, cols_b, b_rpt, b_col, b_val, b_nnz};
         long long nnz = 0;
         h->op_dtype = dtype;
         h->op_aval = a_val;
