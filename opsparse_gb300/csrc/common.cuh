@@ -128,6 +128,7 @@ struct DevInfo {
     int e1_size[3];               // E1 rows by shape (e1_shape)
     int e2_size[2];               // E2 rows of the mid and the large shape
     int e1_chain;                 // E1 rows whose A row the next row of A repeats, moved by one column
+    int e1_runs;                  // runs of such rows, cut at every 32 rows
     int groups;                   // groups of rows of one pattern (regular.cuh)
     unsigned long long d_len_a;   // A entries of the D rows
     unsigned long long d_flop;    // products of the D rows

@@ -107,6 +107,7 @@ struct ops_handle_s {
     int e1_size[3] = {}, e2_size[2] = {};  // E1 and E2 rows by shape (DevInfo)
     bool small = false;           // one kernel takes every row (k_rank_all)
     bool regular = false;         // some E1 rows are in groups of one pattern (regular.cuh)
+    bool no_groups = false;       // ... could have been: the host knows that none are
     long long plan_flop = 0;
     long long plan_nnz = 0;
     int d_rows_path[2] = {};      // D rows of the last phase by [whole-GPU sort, dense kernel]

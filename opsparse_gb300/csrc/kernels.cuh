@@ -86,6 +86,7 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
     __shared__ int s_e1one;
     __shared__ int s_size[5];
     __shared__ int s_chained;
+    __shared__ int s_runs;
     __shared__ int s_huge_rows;
     __shared__ int2 s_huge[kSetupHugeRows];  // A entries of the CTA's longest rows
     __shared__ unsigned long long s_huge_flop[kSetupHugeRows];
@@ -107,6 +108,7 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
         s_huge_rows = 0;
         s_e1one = 0;
         s_chained = 0;
+        s_runs = 0;
         for (int i = 0; i < 5; ++i) s_size[i] = 0;
     }
     __syncthreads();
@@ -397,8 +399,11 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
     }
     chained &= cls == kClsE1;
     if (in) link[r] = chained ? 1 : 0;
-    const int n_chained = __popc(__ballot_sync(kFull, chained));
-    if (lane == 0 && n_chained) atomicAdd(&s_chained, n_chained);
+    const unsigned chain = __ballot_sync(kFull, chained);
+    if (lane == 0 && chain) {
+        atomicAdd(&s_chained, __popc(chain));
+        atomicAdd(&s_runs, __popc(chain & ~(chain << 1)));  // their runs, cut at every 32 rows
+    }
     const unsigned long long wsf = warp_sum_u64((unsigned long long)staged);
     unsigned long long wf = warp_sum_u64((unsigned long long)flop);
     const unsigned wsmall = __reduce_add_sync(kFull, small_nnz);
@@ -420,7 +425,10 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
         for (int w = 0; w < kSetupThreads / 32; ++w) ts += s_sflop[w];
         if (ts) atomicAdd(&info->staged_flop, ts);
         if (s_e1one) atomicAdd(&info->e1_one, s_e1one);
-        if (s_chained) atomicAdd(&info->e1_chain, s_chained);
+        if (s_chained) {
+            atomicAdd(&info->e1_chain, s_chained);
+            atomicAdd(&info->e1_runs, s_runs);
+        }
         for (int i = 0; i < 5; ++i)
             if (s_size[i]) atomicAdd(i < 3 ? &info->e1_size[i] : &info->e2_size[i - 3], s_size[i]);
         unsigned long long sn = 0;

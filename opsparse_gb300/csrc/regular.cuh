@@ -35,7 +35,10 @@ namespace opsg {
 
 constexpr int kGroupRows = 256;     // rows of a group, at most
 constexpr int kGroupLanes = 32;     // rows computed together: a lane each
-constexpr int kGroupMin = 6;        // shorter runs stay with their class
+// Runs of fewer rows stay with their class: on runs of 17 rows a 60x60x19 grid took 572 us
+// grouped and 537 hashed (FP64, two phases), on runs of 28 rows a 30^3 grid 276 and 345.
+constexpr int kGroupMin = 20;
+constexpr int kGroupRestMin = 6;    // rows after the last 32 of a run that still join its group
 constexpr int kGroupAMax = 32;      // A entries of a grouped row: a bit each in an entry's mask
 constexpr int kGroupWindow = 1024;  // rows whose runs one warp cuts
 constexpr int kGroupStage = 9216;   // B values staged for 32 rows, at most
@@ -136,7 +139,7 @@ static __global__ void __launch_bounds__(128) k_form_groups(int M, unsigned char
         const int e = 32 * we + __ffs(__shfl_sync(kFull, m, we)) - 1;
         const int len = e - s + 1;
         const int rest = len % kGroupLanes;
-        const int grouped = len - (rest < kGroupMin ? rest : 0);
+        const int grouped = len < kGroupMin ? 0 : len - (rest < kGroupRestMin ? rest : 0);
         const int n = (grouped + kGroupRows - 1) / kGroupRows;
         if (n > 0) {
             int base = 0;
@@ -400,7 +403,7 @@ __global__ void __launch_bounds__(kGroupThreads, 2) k_group_rows(SpgemmArgs<T> g
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        stage(0, min(gr.y, kGroupLanes));
+        stage(0, gr.y > 24 ? min(kGroupLanes, gr.y) : min(16, gr.y));
         // the pattern: products' columns, entries and positions
         unsigned col[PER], idx[PER];
         int own[PER], at[PER];
@@ -462,8 +465,11 @@ __global__ void __launch_bounds__(kGroupThreads, 2) k_group_rows(SpgemmArgs<T> g
         if (t == 0) s.start[total] = (unsigned)products;
         const bool fits = __ldg(g.c_rpt + gr.x + gr.y) - off == gr.y * total;
         if (t == 0 && !fits) atomicOr(&g.info->flags, kErrCountMismatch);
-        for (int r0 = 0; r0 < gr.y; r0 += kGroupLanes) {
-            const int n = min(kGroupLanes, gr.y - r0);
+        int n = 0;
+        for (int r0 = 0; r0 < gr.y; r0 += n) {
+            // 17 to 24 rows as 16 and the rest: three quarters of the FMAs of a 32-row walk
+            const int rest = gr.y - r0;
+            n = rest > 24 ? min(kGroupLanes, rest) : min(16, rest);
             if (r0 > 0) stage(r0, n);
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();

@@ -341,17 +341,19 @@ int launch_staged_class(ops_handle_s *h, const GA &gs, int c, const int *list, i
     return OPS_OK;
 }
 
-// Below this many rows that the next row of A may continue, the groups' four extra launches
-// (about 15 us) are not worth it: a row saves about 4 ns (61x47x53 grid, FP32: 0.27 ms for
-// 150,000 rows), so the sides meet at about 4,000 rows.
-constexpr int kMinChainRows = 4096;
+// Rows that the next row of A repeats from which the groups' five extra launches (about 35 us
+// of a two-phase call) pay: 27-point operators of a 27^3 grid (17,000 such rows) 255 us
+// grouped against 242, of 30^3 (25,000) 276 against 345.  Short runs do not: k_setup counts
+// them cut at every 32 rows, where runs of 28 rows average 14 and of 17 rows 11.
+constexpr int kMinChainRows = 20480;
+constexpr int kMinChainRun = 14;
 
 // Groups of rows of one pattern (regular.cuh), where k_setup found enough E1 rows that A's
 // next row repeats: links from B, groups, and the E1 rows outside them (h->regular).
 int form_groups(ops_handle_s *h, const DevInfo &hi, const Mat &A, const Mat &B, cudaStream_t st)
 {
     h->regular = false;
-    if (hi.e1_chain < kMinChainRows) return OPS_OK;
+    if (hi.e1_chain < kMinChainRows || hi.e1_chain < kMinChainRun * hi.e1_runs) return OPS_OK;
     const int M = A.rows, K = A.cols;
     if (h->b_link_rows < K) {
         if (h->b_link) OPS_CUDA(h, cudaFreeAsync(h->b_link, st));
@@ -500,7 +502,7 @@ int launch_classes(ops_handle_s *h, const SpgemmArgs<T> &g, cudaStream_t st)
             ++h->launches;
         }
         if (h->timing >= 2) OPS_CUDA(h, cudaEventRecord(h->ev_k[kNum][c][0], s));
-        if (c == kClsE1 && h->regular) {  // the groups of one pattern, then the class's other rows
+        if (c == kClsE1 && h->regular && !(kNum && h->no_groups)) {  // the groups of one pattern, then the other rows
             OPS_CHECK((launch_groups<kNum, T>(h, g, n, s)));
         }
         if (staged && !kNum) {  // one-pass call: numeric into the staging area
@@ -762,6 +764,7 @@ int run_symbolic(ops_handle_s *h, const Mat &A, const Mat &B, int *c_rpt, long l
     h->staged = false;
     h->small = small;
     h->regular = false;
+    h->no_groups = false;
     h->plan_arpt = A.rpt;
     h->plan_acol = A.col;
     h->plan_brpt = B.rpt;
@@ -792,6 +795,7 @@ int run_symbolic(ops_handle_s *h, const Mat &A, const Mat &B, int *c_rpt, long l
         OPS_CHECK(count_status(h, h2));
         *c_nnz = (long long)h2.total_nnz;
         h->plan_nnz = (long long)h2.total_nnz;
+        h->no_groups = h2.groups == 0;
     }
     h->plan_valid = true;
     return OPS_OK;

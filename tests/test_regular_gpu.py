@@ -45,11 +45,13 @@ def banded(name, rows, cuts, seed):
     return build(rows, offs_a, cut_a), build(k, offs_b, cut_b), ncols
 
 
-@pytest.mark.parametrize("name,rows,cuts", [("stencil25", 6000, 0), ("stencil25", 9000, 300), ("one_pencil", 5001, 150),
-                                            ("short", 20000, 1500), ("odd_pencils", 9001, 40),
-                                            ("odd_pencils", 6003, 900), ("pencils", 6000, 20), ("short", 1000, 10)])
+@pytest.mark.parametrize("name,rows,cuts,groups", [("stencil25", 25000, 0, True), ("stencil25", 30000, 350, True),
+                                                   ("one_pencil", 25001, 300, True), ("short", 60000, 1000, True),
+                                                   ("odd_pencils", 30001, 40, True), ("odd_pencils", 33003, 600, True),
+                                                   ("pencils", 25000, 20, False), ("short", 1000, 10, False),
+                                                   ("short", 40000, 6000, False)])
 @pytest.mark.parametrize("dtype", ["f64", "f32"])
-def test_groups_of_one_pattern(cuda, dtype, name, rows, cuts):
+def test_groups_of_one_pattern(cuda, dtype, name, rows, cuts, groups):
     torch = cuda
     npdt = np.float64 if dtype == "f64" else np.float32
     tdt = torch.float64 if dtype == "f64" else torch.float32
@@ -70,7 +72,7 @@ def test_groups_of_one_pattern(cuda, dtype, name, rows, cuts):
         c_col, c_val = h.numeric(A, B, c_rpt, nnz)
         same(c_rpt.cpu().numpy(), c_col.cpu().numpy(), c_val.cpu().numpy(), oval)
         grouped = rows - sum(h.subclass_rows()[k] for k in ("e1_sort", "e1_hash", "e1_esc"))
-        assert (grouped > rows // 3) == (name != "pencils" and rows > 4096), grouped
+        assert (grouped > rows // 4) == groups, grouped
         h.set_one_pass(2)
         same(*h.spgemm_oneshot(A, B).to_host(), oval)
         rng = np.random.default_rng(5)
