@@ -17,6 +17,10 @@
 //               enumeration = exclusive scan of the B-row lengths over A's entries;
 //   at_ptr/at_ent  A's entries ordered by (column, row): CUB radix sort by column, which
 //               is stable, over entries in row-major order;
+//   at_src[e]   what the e-th of them needs to find its products' positions in C: the index
+//               of its first product (with the map below), else its row;
+//   brow[q]     row of B entry q;
+//   long_b      the chunks of B entries whose column of A is long (k_grad_b_long);
 //   pmap[q]     position in C of product q, found once by binary search in C's sorted
 //               row — only when products * 4 bytes fits the handle's map budget.  Without
 //               it every product's position is searched again on each call.
@@ -24,6 +28,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "common.cuh"
 #include "internal.hpp"
@@ -32,6 +37,9 @@ using namespace opsg;
 using namespace opsg_internal;
 
 namespace {
+
+constexpr int kGradBatch = 8;      // chain steps whose operands are loaded together
+constexpr int kGradShortMax = 64;  // chains longer than this are folded by a warp
 
 // First index in a[0, n) with a[idx] >= key.
 __device__ __forceinline__ int lower_bound_i32(const int *__restrict__ a, int n, int key)
@@ -74,14 +82,14 @@ __global__ void k_iota(int *out, long long n)
         out[p] = (int)p;
 }
 
-// arow[p] = row of A entry p; one warp per row.
-__global__ void k_expand_rows(const int *__restrict__ arpt, int M, int *__restrict__ arow)
+// arow[p] = row of entry p < nnz; one warp per row.
+__global__ void k_expand_rows(const int *__restrict__ arpt, int M, long long nnz, int *__restrict__ arow)
 {
     const long long w0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
     for (long long i = w0; i < M; i += nw) {
         const int a0 = __ldg(arpt + i), a1 = __ldg(arpt + i + 1);
-        for (int p = a0 + lane_id(); p < a1; p += 32) arow[p] = (int)i;
+        for (int p = a0 + lane_id(); p < a1 && p < nnz; p += 32) arow[p] = (int)i;
     }
 }
 
@@ -92,6 +100,29 @@ __global__ void k_col_starts(const int *__restrict__ sorted_cols, long long nnz,
         const int cur = p < nnz ? __ldg(sorted_cols + p) : K;
         const int prev = p > 0 ? __ldg(sorted_cols + p - 1) : -1;
         for (int j = prev + 1; j <= cur; ++j) at_ptr[j] = (int)p;
+    }
+}
+
+// The chunks of up to 32 entries of one row of B whose column of A is too long for a thread
+// (k_grad_b_long); their order does not matter to the results.
+__global__ void k_list_long_b(long long nnz_b, const int *__restrict__ brow, const int *__restrict__ brpt,
+                              const int *__restrict__ at_ptr, int *__restrict__ list, int *count)
+{
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nnz_b; q += (long long)gridDim.x * blockDim.x) {
+        const int j = __ldg(brow + q);
+        if (__ldg(at_ptr + j + 1) - __ldg(at_ptr + j) > kGradShortMax && (q - __ldg(brpt + j)) % 32 == 0)
+            list[atomicAdd(count, 1)] = (int)q;
+    }
+}
+
+// at_src[e]: first product of the e-th column-ordered A entry (with a map), else its row.
+template <bool kMap>
+__global__ void k_column_sources(const int *__restrict__ at_ent, long long nnz, const long long *__restrict__ pos_base,
+                                 const int *__restrict__ arow, int *__restrict__ at_src)
+{
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nnz; e += (long long)gridDim.x * blockDim.x) {
+        const int p = __ldg(at_ent + e);
+        at_src[e] = kMap ? (int)__ldg(pos_base + p) : __ldg(arow + p);
     }
 }
 
@@ -127,9 +158,6 @@ __device__ __forceinline__ int prod_pos(const int *__restrict__ pmap, long long 
     if constexpr (kMap) return __ldg(pmap + base + t);
     return c_position(c_rpt, c_col, i, key, flags);
 }
-
-constexpr int kGradBatch = 8;      // chain steps whose operands are loaded together
-constexpr int kGradShortMax = 64;  // dA chains longer than this are folded by a warp
 
 // dA, chains of at most kGradShortMax terms: one thread per A entry p = (i, j), folding
 // B row j in order, kGradBatch terms' operands loaded ahead of their FMAs.  Longer chains
@@ -235,63 +263,107 @@ __global__ void __launch_bounds__(256) k_grad_a_long(const int *__restrict__ aco
     }
 }
 
-// dB: one warp per row j of B, lanes over the row's entries q, each folding the A entries
-// of column j in ascending row order.  All lanes walk the same column entries, so the
-// warp loads 32 of them at once (one per lane) and shares them by shuffle; each lane then
-// loads kGradBatch terms' positions and dC values ahead of its FMAs.
+// dB, columns of A with at most kGradShortMax entries: one thread per B entry q = (j, k),
+// folding the A entries of column j in ascending row order, kGradBatch terms' operands
+// loaded ahead of their FMAs.  The threads of one row of B read the same column entries (one
+// request each) and neighbouring positions.  Bound by the gathers of dC, a 32-byte sector a
+// product: a warp per row of B left the lanes beyond the row's length idle, and took one
+// dependent load more to find each product's position.
 template <typename T, bool kMap>
-__global__ void __launch_bounds__(256) k_grad_b(int K, const int *__restrict__ brpt, const int *__restrict__ bcol,
-                                                 const T *__restrict__ aval, const int *__restrict__ at_ptr,
-                                                 const int *__restrict__ at_ent, const int *__restrict__ arow,
-                                                 const int *__restrict__ c_rpt, const int *__restrict__ c_col,
-                                                 const T *__restrict__ dc, const long long *__restrict__ pos_base,
-                                                 const int *__restrict__ pmap, T *__restrict__ db, int *flags)
+__global__ void __launch_bounds__(256) k_grad_b_short(long long nnz_b, const int *__restrict__ brow,
+                                                       const int *__restrict__ brpt, const int *__restrict__ bcol,
+                                                       const T *__restrict__ aval, const int *__restrict__ at_ptr,
+                                                       const int *__restrict__ at_ent, const int *__restrict__ at_src,
+                                                       const int *__restrict__ c_rpt, const int *__restrict__ c_col,
+                                                       const T *__restrict__ dc, const int *__restrict__ pmap,
+                                                       T *__restrict__ db, int *flags)
+{
+    using AccT = Acc<T>;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nnz_b;
+         q += (long long)gridDim.x * blockDim.x) {
+        const int j = __ldg(brow + q);
+        const int e0 = __ldg(at_ptr + j), e1 = __ldg(at_ptr + j + 1);
+        if (e1 - e0 > kGradShortMax) continue;  // k_grad_b_long's
+        const int t = (int)(q - __ldg(brpt + j));
+        const int key = kMap ? 0 : __ldg(bcol + q);
+        typename AccT::S s = AccT::zero();
+        for (int eb = e0; eb < e1; eb += kGradBatch) {
+            int pos[kGradBatch];
+            T a[kGradBatch], d[kGradBatch];
+#pragma unroll
+            for (int u = 0; u < kGradBatch; ++u) {
+                pos[u] = -1;
+                a[u] = T(0);
+                if (eb + u < e1) {
+                    const int src = __ldg(at_src + eb + u);
+                    a[u] = __ldg(aval + __ldg(at_ent + eb + u));
+                    pos[u] = prod_pos<kMap>(pmap, src, t, c_rpt, c_col, src, key, flags);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kGradBatch; ++u) d[u] = pos[u] >= 0 ? __ldg(dc + pos[u]) : T(0);
+#pragma unroll
+            for (int u = 0; u < kGradBatch; ++u)
+                if (eb + u < e1) s = AccT::step(s, a[u], d[u]);
+        }
+        db[q] = AccT::fin(s);
+    }
+}
+
+// dB, longer columns: one warp per listed chunk of up to 32 entries of one row j of B, lanes
+// over the entries q, each folding the A entries of column j in ascending row order.  All
+// lanes walk the same column entries, so the warp loads 32 of them at once (one per lane) and
+// shares them by shuffle; each lane then loads kGradBatch terms' positions and dC values
+// ahead of its FMAs.
+template <typename T, bool kMap>
+__global__ void __launch_bounds__(256) k_grad_b_long(const int *__restrict__ list, int count,
+                                                      const int *__restrict__ brow, const int *__restrict__ brpt,
+                                                      const int *__restrict__ bcol, const T *__restrict__ aval,
+                                                      const int *__restrict__ at_ptr, const int *__restrict__ at_ent,
+                                                      const int *__restrict__ at_src, const int *__restrict__ c_rpt,
+                                                      const int *__restrict__ c_col, const T *__restrict__ dc,
+                                                      const int *__restrict__ pmap, T *__restrict__ db, int *flags)
 {
     using AccT = Acc<T>;
     const int lane = lane_id();
     const long long w0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long j = w0; j < K; j += nw) {
+    for (long long it = w0; it < count; it += nw) {
+        const int qb = __ldg(list + it);
+        const int j = __ldg(brow + qb);
         const int b0 = __ldg(brpt + j), b1 = __ldg(brpt + j + 1);
         const int e0 = __ldg(at_ptr + j), e1 = __ldg(at_ptr + j + 1);
-        for (int qb = b0; qb < b1; qb += 32) {
-            const int q = qb + lane;
-            const bool qv = q < b1;
-            const int key = (!kMap && qv) ? __ldg(bcol + q) : 0;
-            typename AccT::S s = AccT::zero();
-            for (int eb = e0; eb < e1; eb += 32) {
-                // one column entry per lane: its A entry, row, value and product base
-                int pe = 0, re = 0;
-                long long be = 0;
-                T ae = T(0);
-                if (eb + lane < e1) {
-                    pe = __ldg(at_ent + eb + lane);
-                    ae = __ldg(aval + pe);
-                    if (kMap) be = __ldg(pos_base + pe);
-                    else re = __ldg(arow + pe);
-                }
-                const int m = min(32, e1 - eb);
-                for (int t0 = 0; t0 < m; t0 += kGradBatch) {
-                    int pos[kGradBatch];
-                    T a[kGradBatch], d[kGradBatch];
-#pragma unroll
-                    for (int u = 0; u < kGradBatch; ++u) {
-                        const int src = min(t0 + u, 31);
-                        const long long bu = kMap ? __shfl_sync(kFull, be, src) : 0;
-                        const int ru = kMap ? 0 : __shfl_sync(kFull, re, src);
-                        a[u] = shfl(ae, src);
-                        pos[u] = (qv && t0 + u < m) ? prod_pos<kMap>(pmap, bu, q - b0, c_rpt, c_col, ru, key, flags)
-                                                    : -1;
-                    }
-#pragma unroll
-                    for (int u = 0; u < kGradBatch; ++u) d[u] = pos[u] >= 0 ? __ldg(dc + pos[u]) : T(0);
-#pragma unroll
-                    for (int u = 0; u < kGradBatch; ++u)
-                        if (t0 + u < m) s = AccT::step(s, a[u], d[u]);
-                }
+        const int q = qb + lane;
+        const bool qv = q < b1;
+        const int key = (!kMap && qv) ? __ldg(bcol + q) : 0;
+        typename AccT::S s = AccT::zero();
+        for (int eb = e0; eb < e1; eb += 32) {
+            // one column entry per lane: its value, and its product base or its row
+            int se = 0;
+            T ae = T(0);
+            if (eb + lane < e1) {
+                se = __ldg(at_src + eb + lane);
+                ae = __ldg(aval + __ldg(at_ent + eb + lane));
             }
-            if (qv) db[q] = AccT::fin(s);
+            const int m = min(32, e1 - eb);
+            for (int t0 = 0; t0 < m; t0 += kGradBatch) {
+                int pos[kGradBatch];
+                T a[kGradBatch], d[kGradBatch];
+#pragma unroll
+                for (int u = 0; u < kGradBatch; ++u) {
+                    const int lu = min(t0 + u, 31);
+                    const int su = __shfl_sync(kFull, se, lu);
+                    a[u] = shfl(ae, lu);
+                    pos[u] = (qv && t0 + u < m) ? prod_pos<kMap>(pmap, su, q - b0, c_rpt, c_col, su, key, flags) : -1;
+                }
+#pragma unroll
+                for (int u = 0; u < kGradBatch; ++u) d[u] = pos[u] >= 0 ? __ldg(dc + pos[u]) : T(0);
+#pragma unroll
+                for (int u = 0; u < kGradBatch; ++u)
+                    if (t0 + u < m) s = AccT::step(s, a[u], d[u]);
+            }
         }
+        if (qv) db[q] = AccT::fin(s);
     }
 }
 
@@ -341,8 +413,10 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
     void *scan_scratch = t;
 
     // persistent plan arrays (map added below once the product count is known)
+    const size_t nb = (size_t)std::max<long long>(nnz_b, 1);
+    const size_t list_b = na / kGradShortMax + nb / 32 + 1;  // a chunk a listed row, and one per 32 entries
     const size_t base_bytes = align_up(8 * (na + 1), 256) + align_up(4 * ((size_t)K + 1), 256) +
-                              align_up(4 * na, 256) * 2;
+                              align_up(4 * na, 256) * 3 + align_up(4 * nb, 256) + align_up(4 * list_b, 256);
     void *pp = nullptr;
     OPS_CUDA(h, cudaMallocFromPoolAsync(&pp, base_bytes, h->pool, st));
     unsigned char *m = static_cast<unsigned char *>(pp);
@@ -355,6 +429,12 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
     pl.at_ent = reinterpret_cast<int *>(m);
     m += align_up(4 * na, 256);
     pl.arow = reinterpret_cast<int *>(m);
+    m += align_up(4 * na, 256);
+    pl.at_src = reinterpret_cast<int *>(m);
+    m += align_up(4 * na, 256);
+    pl.brow = reinterpret_cast<int *>(m);
+    m += align_up(4 * nb, 256);
+    pl.long_b = reinterpret_cast<int *>(m);
 
     OPS_CUDA(h, cudaMemsetAsync(blen + na, 0, sizeof(long long), st));
     if (nnz_a > 0) {
@@ -364,7 +444,7 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
     }
     OPS_CUDA(h, cub::DeviceScan::ExclusiveSum(scan_scratch, scan_tmp, blen, pl.pos_base, (int)na + 1, st));
     if (M > 0) {
-        k_expand_rows<<<grid_of(M, 8, sms * 8), 256, 0, st>>>(a_rpt, M, pl.arow);
+        k_expand_rows<<<grid_of(M, 8, sms * 8), 256, 0, st>>>(a_rpt, M, nnz_a, pl.arow);
         OPS_CUDA(h, cudaGetLastError());
     }
     if (nnz_a > 0)
@@ -372,6 +452,14 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
                                                     (int)nnz_a, 0, std::max(1, ceil_log2(std::max(K, 2))), st));
     k_col_starts<<<grid_of(nnz_a + 1, 256, sms * 16), 256, 0, st>>>(sorted_cols, nnz_a, K, pl.at_ptr);
     OPS_CUDA(h, cudaGetLastError());
+    OPS_CUDA(h, cudaMemsetAsync(&h->info->d_cursor, 0, sizeof(int), st));
+    if (nnz_b > 0) {
+        k_expand_rows<<<grid_of(K, 8, sms * 8), 256, 0, st>>>(b_rpt, K, nnz_b, pl.brow);
+        k_list_long_b<<<grid_of(nnz_b, 256, sms * 16), 256, 0, st>>>(nnz_b, pl.brow, b_rpt, pl.at_ptr, pl.long_b,
+                                                                     &h->info->d_cursor);
+        OPS_CUDA(h, cudaGetLastError());
+    }
+    OPS_CUDA(h, cudaMemcpyAsync(&pl.long_b_count, &h->info->d_cursor, sizeof(int), cudaMemcpyDeviceToHost, st));
     long long products = 0;
     OPS_CUDA(h, cudaMemcpyAsync(&products, pl.pos_base + na - (nnz_a > 0 ? 0 : 1), sizeof(long long),
                                 cudaMemcpyDeviceToHost, st));
@@ -393,6 +481,12 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
             (void)cudaGetLastError();
             pl.with_map = false;  // no room: search positions on every call instead
         }
+    }
+    if (nnz_a > 0) {
+        const int g = grid_of(nnz_a, 256, sms * 16);
+        if (pl.with_map) k_column_sources<true><<<g, 256, 0, st>>>(pl.at_ent, nnz_a, pl.pos_base, pl.arow, pl.at_src);
+        else k_column_sources<false><<<g, 256, 0, st>>>(pl.at_ent, nnz_a, pl.pos_base, pl.arow, pl.at_src);
+        OPS_CUDA(h, cudaGetLastError());
     }
     OPS_CUDA(h, cudaFreeAsync(tp, st));
     pl.M = M;
@@ -442,15 +536,19 @@ int run_backward(ops_handle_s *h, int M, int K, const int *a_rpt, const int *a_c
         OPS_CUDA(h, cudaGetLastError());
         OPS_CUDA(h, cudaFreeAsync(long_list, st));
     }
-    if (db && K > 0) {
-        if (pl.with_map)
-            k_grad_b<T, true><<<grid_of(K, 8, sms * 8), 256, 0, st>>>(K, b_rpt, b_col, a_val, pl.at_ptr, pl.at_ent,
-                                                                      pl.arow, c_rpt, c_col, dc, pl.pos_base, pl.pmap,
-                                                                      db, flags);
-        else
-            k_grad_b<T, false><<<grid_of(K, 8, sms * 8), 256, 0, st>>>(K, b_rpt, b_col, a_val, pl.at_ptr, pl.at_ent,
-                                                                       pl.arow, c_rpt, c_col, dc, pl.pos_base, pl.pmap,
-                                                                       db, flags);
+    if (db && pl.nnz_b > 0) {
+        const int g1 = grid_of(pl.nnz_b, 256, sms * 16), g2 = grid_of(pl.long_b_count, 8, sms * 8);
+        auto launch = [&](auto map) {
+            constexpr bool kMap = decltype(map)::value;
+            k_grad_b_short<T, kMap><<<g1, 256, 0, st>>>(pl.nnz_b, pl.brow, b_rpt, b_col, a_val, pl.at_ptr, pl.at_ent,
+                                                        pl.at_src, c_rpt, c_col, dc, pl.pmap, db, flags);
+            if (pl.long_b_count > 0)
+                k_grad_b_long<T, kMap><<<g2, 256, 0, st>>>(pl.long_b, pl.long_b_count, pl.brow, b_rpt, b_col, a_val,
+                                                           pl.at_ptr, pl.at_ent, pl.at_src, c_rpt, c_col, dc, pl.pmap,
+                                                           db, flags);
+        };
+        if (pl.with_map) launch(std::true_type{});
+        else launch(std::false_type{});
         OPS_CUDA(h, cudaGetLastError());
     }
     return OPS_OK;

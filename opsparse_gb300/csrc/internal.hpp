@@ -28,6 +28,10 @@ struct BackwardPlan {
     int *at_ptr = nullptr;          // [K+1] columns of A (transpose row pointers)
     int *at_ent = nullptr;          // [nnz_a] A entries ordered by (column, row)
     int *arow = nullptr;            // [nnz_a] row of each A entry
+    int *at_src = nullptr;          // [nnz_a] first product (with a map) or row of each column-ordered A entry
+    int *brow = nullptr;            // [nnz_b] row of each B entry
+    int *long_b = nullptr;          // first entries of the chunks of B rows whose column of A is long
+    int long_b_count = 0;
 };
 
 struct ops_handle_s {
