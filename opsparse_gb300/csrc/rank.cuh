@@ -21,8 +21,8 @@
 //                bit already set);
 //   numeric:  4. a product whose column is not repeated is its entry.  The products of
 //                repeated columns fold in product order, 32 at a time, those of one A entry
-//                in one step (a B row holds a column once); a CTA lists them first and
-//                each warp takes its share of the positions.  One FMA per product, the
+//                in one step (a B row holds a column once); a CTA lists them first, by the
+//                warp that folds their position.  One FMA per product, the
 //                oracle's sequence bit for bit;
 //             5. C's row is written in column order from shared memory.
 //
@@ -47,7 +47,7 @@ namespace opsg {
 // in registers from the expansion on.
 template <int NT, int PER, int ACAP, int GROUPS, int MINB, int TOP, bool RELOAD64 = false>
 struct RankShape {
-    static_assert(NT % 32 == 0 && (GROUPS == 1 || NT == 32), "rows of several warps take a whole CTA");
+    static_assert((NT & (NT - 1)) == 0 && NT >= 32 && (GROUPS == 1 || NT == 32), "rows of several warps take a whole CTA");
     static constexpr int kGroup = NT;
     static constexpr int kPer = PER;
     static constexpr int kGroups = GROUPS;
@@ -72,7 +72,7 @@ struct RankShape {
     static constexpr size_t cmax(size_t a, size_t b) { return a > b ? a : b; }
     // [B offset | A value (wide: A position) | first product per entry] [chunk table] [scan]
     // [repeated positions] [wide: their prefixes] [levels; later: values | columns by
-    // position | list of products, their entries and positions]
+    // position | list of products, their entries and positions | counts]
     static constexpr size_t kOffAt = 0;
     static constexpr size_t kAvalAt = kOffAt + up16(4 * (size_t)ACAP);
     static constexpr size_t kStartAt = kAvalAt + up16((kWide ? 4 : 8) * (size_t)ACAP);
@@ -85,10 +85,18 @@ struct RankShape {
     static constexpr size_t kLevelBytes = 8 * ((size_t)kLevel0 + (size_t)kCap);
     static constexpr size_t kColumnAt = kRegionAt + (kWide ? 4 : 8) * (size_t)kCap;
     static constexpr size_t kListAt = kColumnAt + (kWide ? 0 : 4 * (size_t)kCap);
+    // counts of listed products per warp that folds them and chunk; an odd number of words
+    // between warps keeps a chunk's counts in different banks
+    // a listed product, its entry and its position share a word where 10, 12 and 10 bits do
+    static constexpr bool kPacked = kCap <= 1024;
+    static constexpr size_t kCountAt = kListAt + (kPacked ? 4 : 6) * (size_t)kCap;
+    static constexpr int kCountStride = PER * kWarps + 2;
+    static_assert(NT == 32 || PER * kWarps % 4 == 0, "an odd number of words");
     template <bool kNum>
     static constexpr size_t group_bytes()
     {
-        return cmax(kRegionAt + kLevelBytes, kNum ? kListAt + (NT > 32 ? 6 * (size_t)kCap : 0) : 0);
+        return cmax(kRegionAt + kLevelBytes,
+                    kNum ? (NT > 32 ? kCountAt + up16(2 * (size_t)kWarps * kCountStride) : kListAt) : 0);
     }
     template <bool kNum>
     static constexpr size_t smem()
@@ -156,12 +164,14 @@ struct RankSmem {
     __device__ __forceinline__ static int words(int l) { return second(l) ? Sh::kCap : Sh::kLevel0; }
     __device__ __forceinline__ S *val() const { return at<S>(Sh::kRegionAt); }
     __device__ __forceinline__ int *column() const { return at<int>(Sh::kColumnAt); }
-    // listed products: number | entry << 16, and position
+    // listed products: number | entry << 10 | position << 22, or number | entry << 16 and the
+    // position apart
     __device__ __forceinline__ unsigned *list() const { return at<unsigned>(Sh::kListAt); }
     __device__ __forceinline__ unsigned short *list_pos() const
     {
         return at<unsigned short>(Sh::kListAt + 4 * (size_t)Sh::kCap);
     }
+    __device__ __forceinline__ unsigned short *counts() const { return at<unsigned short>(Sh::kCountAt); }
     __device__ __forceinline__ T a_value(const SpgemmArgs<T> &g, int e) const
     {
         if constexpr (Sh::kWide) return __ldg(g.aval + at<int>(Sh::kAvalAt)[e]);
@@ -557,21 +567,38 @@ __device__ __forceinline__ void rank_row(const SpgemmArgs<T> &g, int r, const Ra
                 }
             }
         } else if (n_late > 0) {
-            // listed products in product order: a count per chunk, their prefix, the list
-            unsigned short *tile = sm.first();  // the chunk table is done with
+            // Listed products by the warp that folds them (the low bits of their position), in
+            // product order: a count per warp and chunk, their prefixes, the list.  The lanes
+            // of a chunk that share a warp come from a ballot per bit; the same ballots give
+            // lane w the products of warp w.  (With one list that every warp walked for its
+            // share a row's listing cost as many walks as it has warps: the 40 longest rows of
+            // a web graph 72 -> 43 us, graph of 200,000 nodes times its transpose 2.51 -> 2.37
+            // ms.)
+            unsigned short *counts = sm.counts();
+            auto by_warp = [&](bool in, unsigned pos, unsigned &same, unsigned &lanes) {
+                same = lanes = __ballot_sync(kFull, in);
+#pragma unroll
+                for (int i = 0; (1 << i) < NW; ++i) {
+                    const unsigned m = __ballot_sync(kFull, (pos >> i) & 1u);
+                    same &= ((pos >> i) & 1u) ? m : ~m;
+                    lanes &= ((lane >> i) & 1) ? m : ~m;
+                }
+            };
 #pragma unroll
             for (int k = 0; k < PER; ++k) {
-                const unsigned m = __ballot_sync(kFull, (listed >> k) & 1u);
-                if (lane == 0) tile[k * NW + warp] = (unsigned short)__popc(m);
+                unsigned same, lanes = 0u;
+                if (k * NT + c0 < n) by_warp((listed >> k) & 1u, idx[k], same, lanes);
+                if (lane < NW) counts[lane * Sh::kCountStride + k * NW + warp] = (unsigned short)__popc(lanes);
             }
             __syncthreads();
-            if (warp == 0) {
+            {
                 constexpr int kEach = (PER * NW + 31) / 32;
+                unsigned short *mine = counts + warp * Sh::kCountStride;
                 int v[kEach], sum = 0;
 #pragma unroll
                 for (int i = 0; i < kEach; ++i) {
                     const int q = lane * kEach + i;
-                    v[i] = q < PER * NW ? (int)tile[q] : 0;
+                    v[i] = q < PER * NW ? (int)mine[q] : 0;
                     sum += v[i];
                 }
                 const int incl = warp_incl_scan(sum);
@@ -579,43 +606,60 @@ __device__ __forceinline__ void rank_row(const SpgemmArgs<T> &g, int r, const Ra
 #pragma unroll
                 for (int i = 0; i < kEach; ++i) {
                     const int q = lane * kEach + i;
-                    if (q < PER * NW) tile[q] = (unsigned short)run;
+                    if (q < PER * NW) mine[q] = (unsigned short)run;
                     run += v[i];
                 }
-                if (lane == 31) sm.late()[0] = incl;
+                if (lane == 31) sm.wsum()[warp] = incl;
             }
             __syncthreads();
-            const int items = sm.late()[0];
+            const int held = lane < NW ? sm.wsum()[lane] : 0;
+            const int first = warp_incl_scan(held) - held;  // lane w: warp w's first item
+            const int i_begin = __shfl_sync(kFull, first, warp), i_end = i_begin + __shfl_sync(kFull, held, warp);
             unsigned *list = sm.list();
-            unsigned short *list_pos = sm.list_pos();
+            [[maybe_unused]] unsigned short *list_pos = sm.list_pos();
 #pragma unroll
             for (int k = 0; k < PER; ++k) {
+                if (k * NT + c0 >= n) break;
                 const bool in = (listed >> k) & 1u;
-                const unsigned m = __ballot_sync(kFull, in);
+                unsigned same, lanes;
+                by_warp(in, idx[k], same, lanes);
+                const int w = (int)(idx[k] % NW);
+                const int i = __shfl_sync(kFull, first, w) + __popc(same & lanemask_lt());
                 if (in) {
-                    const int i = tile[k * NW + warp] + __popc(m & lanemask_lt());
-                    list[i] = (unsigned)(t + k * NT) | ((unsigned)own[k] << 16);
-                    list_pos[i] = (unsigned short)idx[k];
+                    const int at = i + counts[w * Sh::kCountStride + k * NW + warp];
+                    const unsigned p = (unsigned)(t + k * NT), x = (unsigned)own[k];
+                    if constexpr (Sh::kPacked) {
+                        list[at] = p | (x << 10) | (idx[k] << 22);
+                    } else {
+                        list[at] = p | (x << 16);
+                        list_pos[at] = (unsigned short)idx[k];
+                    }
                 }
             }
             __syncthreads();
-            // each warp folds the positions of its residue class; the operands of the next
-            // 32 items are loaded ahead
+            // each warp folds its items, the operands of the next 32 loaded ahead
             auto item = [&](int i, unsigned &pos, int &e, T &a, T &b) -> bool {
-                if (i >= items) return false;
-                pos = list_pos[i];
-                if ((int)(pos % NW) != warp) return false;
+                if (i >= i_end) return false;
                 const unsigned x = list[i];
-                e = (int)(x >> 16);
+                unsigned p;
+                if constexpr (Sh::kPacked) {
+                    p = x & 1023u;
+                    e = (int)((x >> 10) & 4095u);
+                    pos = x >> 22;
+                } else {
+                    p = x & 0xffffu;
+                    e = (int)(x >> 16);
+                    pos = list_pos[i];
+                }
                 a = sm.a_value(g, e);
-                b = __ldg(g.bval + sm.off()[e] + (int)(x & 0xffffu));
+                b = __ldg(g.bval + sm.off()[e] + (int)p);
                 return true;
             };
             unsigned pos = 0u, pos_n = 0u;
             int e = 0, e_n = 0;
             T a = T(0), b = T(0), a_n = T(0), b_n = T(0);
-            bool in = item(lane, pos, e, a, b);
-            for (int i0 = 0; i0 < items; i0 += 32) {
+            bool in = item(i_begin + lane, pos, e, a, b);
+            for (int i0 = i_begin; i0 < i_end; i0 += 32) {
                 const bool in_n = item(i0 + 32 + lane, pos_n, e_n, a_n, b_n);
                 rank_fold_positions<T>(in, pos, slot(pos), a, b);
                 in = in_n;
