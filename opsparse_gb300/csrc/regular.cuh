@@ -22,10 +22,12 @@
 //                  remainder of at most 16 or 8 rows takes 2 or 4 entries per warp.
 //
 // What bounds it: FP64 issue (a warp's FMA occupies the SM for about 20 cycles; a 78-row
-// run of the 27-point stencil takes 2.5 FMAs per product, 0.80 ms for an 80^3 grid of the
-// 0.93 ms measured); FP32 instruction issue (the compensated sum and three shared loads a
-// product).  The warp hash, which probes and updates shared memory for every product,
-// took 1.91 ms (FP32, 61x47x53 grid: 548 us against 232), the window count of every row
+// run of the 27-point stencil takes 2.5 FMAs per product, 0.80 ms for an 80^3 grid); FP32
+// instruction issue (83% of the slots; the compensated sum and three shared loads a
+// product).  What is done once a chunk counts as much: with every warp at every pencil of
+// the staging and a search per warp for its share, a 61x47x53 grid took 262 million warp
+// instructions and 268 us in FP32, now 199 million and 216.  The warp hash, which probes and updates shared memory for every product,
+// took 1.91 ms (FP32, 61x47x53 grid: 548 us), the window count of every row
 // 0.58 ms against 0.11 for links, groups and counts.
 #pragma once
 
@@ -44,6 +46,7 @@ constexpr int kGroupWindow = 1024;  // rows whose runs one warp cuts
 constexpr int kGroupStage = 9216;   // B values staged for 32 rows, at most
 constexpr int kGroupThreads = 512;
 constexpr int kGroupFlush = 4;      // entries a warp gathers before it writes them
+constexpr int kGroupParts = kGroupThreads / 8;  // shares of the schedule, at most
 constexpr int kGroupTop = 1024;     // words of the pattern's trie level 0, at most
 
 // b_link[j] = 1 where row j + 1 is row j moved by one column and all its columns are in
@@ -216,16 +219,24 @@ struct GroupSmem {
     int e_base[kGroupAMax];            // and its place in b
     int p_entry[kGroupAMax];           // pencils (runs of entries whose B rows follow one another): first entry
     int p_entries[kGroupAMax];         // and entries
+    int part[kGroupParts + 1];         // first entry at or after each part of the products
     int wsum[32];
     int next;
 };
-static_assert(2 * (sizeof(GroupSmem<double>) + 1024) <= 227 * 1024 && kGroupTop <= kEsc1FlopMax, "two CTAs an SM");
+// CTAs per SM
+template <typename T>
+constexpr int group_ctas()
+{
+    return sizeof(T) == 4 ? 3 : 2;
+}
+static_assert(group_ctas<double>() * (sizeof(GroupSmem<double>) + 1024) <= 227 * 1024 &&
+                  group_ctas<float>() * (sizeof(GroupSmem<float>) + 1024) <= 227 * 1024 && kGroupTop <= kEsc1FlopMax,
+              "the CTAs of an SM fit its shared memory");
 
 // The entries of n rows (n <= SW): part threadIdx.x / SW of the schedule by SW lanes, a lane
 // per row, written to C kGroupFlush entries of a row at a time.
 template <int SW, typename T>
-__device__ __forceinline__ void group_fold(GroupSmem<T> &s, int total, int products, int n, int row0, int pa, int pb,
-                                           int *pc, T *pv)
+__device__ __forceinline__ void group_fold(GroupSmem<T> &s, int total, int n, int row0, int pa, int pb, int *pc, T *pv)
 {
     using AccT = Acc<T>;
     constexpr int kParts = kGroupThreads / SW;
@@ -233,18 +244,7 @@ __device__ __forceinline__ void group_fold(GroupSmem<T> &s, int total, int produ
     const int row = lane % SW;
     const unsigned lanes = SW == 32 ? kFull : ((1u << (SW & 31)) - 1u) << (lane & ~(SW - 1));
     const int part = (int)threadIdx.x / SW;
-    // first entry at or after the part's share of the products
-    auto entry_at = [&](int p) {
-        int lo = 0, hi = total;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if ((int)s.start[mid] < p) lo = mid + 1;
-            else hi = mid;
-        }
-        return lo;
-    };
-    const int o0 = entry_at((int)((long long)products * part / kParts));
-    const int o_end = entry_at((int)((long long)products * (part + 1) / kParts));
+    const int o0 = s.part[part * (kGroupParts / kParts)], o_end = s.part[(part + 1) * (kGroupParts / kParts)];
     int e = (int)s.start[o0];
     const int e_end = (int)s.start[o_end];
     const T *a = s.a + min(row, n - 1) * pa;
@@ -307,7 +307,7 @@ __device__ __forceinline__ void group_fold(GroupSmem<T> &s, int total, int produ
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kGroupThreads, 2) k_group_rows(SpgemmArgs<T> g, const int2 *__restrict__ groups,
+__global__ void __launch_bounds__(kGroupThreads, group_ctas<T>()) k_group_rows(SpgemmArgs<T> g, const int2 *__restrict__ groups,
                                                                  int *cursor)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -382,7 +382,10 @@ __global__ void __launch_bounds__(kGroupThreads, 2) k_group_rows(SpgemmArgs<T> g
             for (int i = warp; i < n; i += NW)
                 if (lane < len_a)
                     copy_async(s.a + i * pa + lane, g.aval + a0 + (long long)(r0 + i) * len_a + lane);
-            for (int q = 0; q < pencils; ++q) {
+            // a pencil by one warp, or by as many as there are to a pencil
+            const int parts = max(1, NW / pencils);
+            for (int w = warp; w < pencils * parts; w += NW) {
+                const int q = w % pencils, part = w / pencils;
                 const int e = s.p_entry[q], rows = s.p_entries[q] - 1 + n, len = s.e_len[e];
                 const T *src = g.bval + s.e_b0[e] + (long long)r0 * len;
                 T *dst = s.b + s.e_base[e];
@@ -390,14 +393,15 @@ __global__ void __launch_bounds__(kGroupThreads, 2) k_group_rows(SpgemmArgs<T> g
                     const int values = rows * len;
                     const int lead = min(values, (int)((kQuad - ((size_t)src / sizeof(T)) % kQuad) % kQuad));
                     const int quads = (values - lead) / kQuad;
-                    for (int i = t; i < quads; i += NT) copy_async16(dst + lead + i * kQuad, src + lead + i * kQuad);
+                    for (int i = part * 32 + lane; i < quads; i += parts * 32)
+                        copy_async16(dst + lead + i * kQuad, src + lead + i * kQuad);
                     const int rest = values - quads * kQuad;  // before and after the whole quads
-                    if (t < rest) {
-                        const int i = t < lead ? t : t + quads * kQuad;
+                    if (part == 0 && lane < rest) {
+                        const int i = lane < lead ? lane : lane + quads * kQuad;
                         copy_async(dst + i, src + i);
                     }
                 } else {
-                    for (int i = warp; i < rows; i += NW)
+                    for (int i = part; i < rows; i += parts)
                         for (int c = lane; c < len; c += 32) copy_async(dst + i * pb + c, src + i * len + c);
                 }
             }
@@ -463,6 +467,16 @@ __global__ void __launch_bounds__(kGroupThreads, 2) k_group_rows(SpgemmArgs<T> g
             }
         }
         if (t == 0) s.start[total] = (unsigned)products;
+        if (t <= kGroupParts) {
+            const int p = (int)((long long)products * t / kGroupParts);
+            int lo = 0, hi = total;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if ((int)s.start[mid] < p) lo = mid + 1;
+                else hi = mid;
+            }
+            s.part[t] = lo;
+        }
         const bool fits = __ldg(g.c_rpt + gr.x + gr.y) - off == gr.y * total;
         if (t == 0 && !fits) atomicOr(&g.info->flags, kErrCountMismatch);
         int n = 0;
@@ -476,9 +490,9 @@ __global__ void __launch_bounds__(kGroupThreads, 2) k_group_rows(SpgemmArgs<T> g
             if (fits) {
                 int *pc = g.c_col + off + r0 * total;
                 T *pv = g.c_val + off + r0 * total;
-                if (n > 16) group_fold<32, T>(s, total, products, n, r0, pa, pb, pc, pv);
-                else if (n > 8) group_fold<16, T>(s, total, products, n, r0, pa, pb, pc, pv);
-                else group_fold<8, T>(s, total, products, n, r0, pa, pb, pc, pv);
+                if (n > 16) group_fold<32, T>(s, total, n, r0, pa, pb, pc, pv);
+                else if (n > 8) group_fold<16, T>(s, total, n, r0, pa, pb, pc, pv);
+                else group_fold<8, T>(s, total, n, r0, pa, pb, pc, pv);
             }
             __syncthreads();  // the staged values are done with
         }
