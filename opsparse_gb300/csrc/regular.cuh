@@ -18,18 +18,23 @@
 //                  products in ascending j, once.  32 rows at a time, A's and B's values are
 //                  staged in shared memory (a B row once for all rows and A entries that
 //                  reach it) and a lane is a row: a warp walks its share of the schedule with
-//                  one FMA per product of 32 rows and the accumulator in a register.  A
-//                  remainder of at most 16 or 8 rows takes 2 or 4 entries per warp.
+//                  one FMA per product of 32 rows and the accumulator in a register (FP32: 64
+//                  rows, two a lane).  A remainder of at most 16 or 8 rows takes 2 or 4
+//                  entries per warp.
 //
 // What bounds it: FP64 issue (a warp's FMA occupies the SM for about 20 cycles; a 78-row
 // run of the 27-point stencil takes 2.5 FMAs per product, 0.80 ms for an 80^3 grid); FP32
-// instruction issue (83% of the slots; the compensated sum and three shared loads a
-// product).  What is done once a chunk counts as much: with every warp at every pencil of
-// the staging and a search per warp for its share, a 61x47x53 grid took 262 million warp
-// instructions and 268 us in FP32, now 199 million and 216.  The warp hash, which probes and updates shared memory for every product,
+// instruction issue (80% of the slots; the compensated sum and three shared loads a
+// product), so a lane takes two rows there and the compensated sums of both in packed
+// instructions: 61x47x53 grid, the numeric phase 331 us against 283.  What is done once a
+// chunk counts as much: with every warp at every pencil of the staging and a search per warp
+// for its share the kernel took 262 million warp instructions and 268 us, without 199
+// million and 216 (a row per lane).  The warp hash, which probes and updates shared memory for every product,
 // took 1.91 ms (FP32, 61x47x53 grid: 548 us), the window count of every row
 // 0.58 ms against 0.11 for links, groups and counts.
 #pragma once
+
+#include <type_traits>
 
 #include "lists.cuh"
 
@@ -201,10 +206,14 @@ __device__ __forceinline__ void copy_async16(T *dst, const T *src)
 
 template <typename T>
 struct GroupSmem {
-    T b[kGroupStage];                           // B values: slot rows of one pitch
-    T a[kGroupLanes * (kGroupAMax + 1)];        // A values, rows of lenA | 1
+    // rows walked together, at most: FP32 takes two per lane where their B values fit
+    static constexpr int kRows = sizeof(T) == 4 ? 2 * kGroupLanes : kGroupLanes;
+    static constexpr int kStage = sizeof(T) == 4 ? 17408 : kGroupStage;
+    T b[kStage];                                // B values: slot rows of one pitch
+    // A values, rows of lenA | 1; of rows r and r + 32 in pairs where a lane takes two
+    alignas(16) T a[kRows * (kGroupAMax + 1)];
     union {
-        T tile[kGroupThreads / 32][kGroupFlush * (kGroupLanes + 4)];  // a warp's entries by (entry, row)
+        T tile[kGroupThreads / 32][kGroupFlush * (kRows + 4)];  // a warp's entries by (entry, row)
         struct {  // while the pattern is worked out
             unsigned bits[2][kEsc1FlopMax];     // trie levels, then the entries' masks of A entries
             unsigned pre[2][kEsc1FlopMax];
@@ -223,23 +232,76 @@ struct GroupSmem {
     int wsum[32];
     int next;
 };
-// CTAs per SM
-template <typename T>
-constexpr int group_ctas()
-{
-    return sizeof(T) == 4 ? 3 : 2;
-}
-static_assert(group_ctas<double>() * (sizeof(GroupSmem<double>) + 1024) <= 227 * 1024 &&
-                  group_ctas<float>() * (sizeof(GroupSmem<float>) + 1024) <= 227 * 1024 && kGroupTop <= kEsc1FlopMax,
+constexpr int kGroupCtas = 2;  // per SM
+static_assert(kGroupCtas * (sizeof(GroupSmem<double>) + 1024) <= 227 * 1024 &&
+                  kGroupCtas * (sizeof(GroupSmem<float>) + 1024) <= 227 * 1024 && kGroupTop <= kEsc1FlopMax,
               "the CTAs of an SM fit its shared memory");
 
-// The entries of n rows (n <= SW): part threadIdx.x / SW of the schedule by SW lanes, a lane
-// per row, written to C kGroupFlush entries of a row at a time.
-template <int SW, typename T>
+// Two rows' FP32 accumulators: Acc<float>'s steps on both at once (the packed instructions
+// round each half as their scalar forms do).
+struct AccPair {
+    unsigned long long x, y;  // running sums, running compensations
+    __device__ __forceinline__ static unsigned long long pack(float lo, float hi)
+    {
+        unsigned long long v;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+        return v;
+    }
+    __device__ __forceinline__ static float2 unpack(unsigned long long v)
+    {
+        float2 f;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+        return f;
+    }
+    __device__ __forceinline__ static unsigned long long add(unsigned long long a, unsigned long long b)
+    {
+        unsigned long long v;
+        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+        return v;
+    }
+    __device__ __forceinline__ static unsigned long long sub(unsigned long long a, unsigned long long b)
+    {
+        unsigned long long v;
+        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+        return v;
+    }
+    __device__ __forceinline__ static unsigned long long mul(unsigned long long a, unsigned long long b)
+    {
+        unsigned long long v;
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+        return v;
+    }
+    __device__ __forceinline__ static unsigned long long fma(unsigned long long a, unsigned long long b,
+                                                             unsigned long long c)
+    {
+        unsigned long long v;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+        return v;
+    }
+    __device__ __forceinline__ void step(unsigned long long a, unsigned long long b)
+    {
+        // TwoProduct: h + r == a*b.  h is negated by its sign bits: with a packed subtraction
+        // from zero in its place the compiled code lost r (tested against the scalar steps).
+        const unsigned long long h = mul(a, b);
+        const unsigned long long r = fma(a, b, h ^ 0x8000000080000000ull);
+        const unsigned long long s = add(x, h);  // TwoSum: s + q == x + h
+        const unsigned long long z = sub(s, x);
+        const unsigned long long q = add(sub(x, sub(s, z)), sub(h, z));
+        x = s;
+        y = add(y, add(q, r));
+    }
+    __device__ __forceinline__ float2 fin() const { return unpack(add(x, y)); }
+};
+
+// The entries of n rows (n <= SW, or 2 * SW in pairs): part threadIdx.x / SW of the schedule
+// by SW lanes, a lane per row or per rows r and r + SW, written to C kGroupFlush entries of a
+// row at a time.
+template <int SW, bool kPair, typename T>
 __device__ __forceinline__ void group_fold(GroupSmem<T> &s, int total, int n, int row0, int pa, int pb, int *pc, T *pv)
 {
     using AccT = Acc<T>;
     constexpr int kParts = kGroupThreads / SW;
+    constexpr int kWidth = kPair ? 2 * SW : SW;  // rows
     const int lane = lane_id();
     const int row = lane % SW;
     const unsigned lanes = SW == 32 ? kFull : ((1u << (SW & 31)) - 1u) << (lane & ~(SW - 1));
@@ -247,9 +309,10 @@ __device__ __forceinline__ void group_fold(GroupSmem<T> &s, int total, int n, in
     const int o0 = s.part[part * (kGroupParts / kParts)], o_end = s.part[(part + 1) * (kGroupParts / kParts)];
     int e = (int)s.start[o0];
     const int e_end = (int)s.start[o_end];
-    const T *a = s.a + min(row, n - 1) * pa;
+    const T *a = s.a + min(row, n - 1) * (kPair ? 2 * pa : pa);
     const T *b = s.b + min(row, n - 1) * pb;
-    T *tile = s.tile[threadIdx.x >> 5] + (lane / SW) * kGroupFlush * (SW + 1);
+    [[maybe_unused]] const T *b1 = s.b + min(row + SW, n - 1) * pb;
+    T *tile = s.tile[threadIdx.x >> 5] + (lane / SW) * kGroupFlush * (kWidth + 1);
     T *put = tile + row;  // this row's next entry
     // the lane's part of a flush: entry fx of rows fr, fr + SW / kGroupFlush, ...
     const int fx = row % kGroupFlush, fr = row / kGroupFlush;
@@ -258,12 +321,12 @@ __device__ __forceinline__ void group_fold(GroupSmem<T> &s, int total, int n, in
     pv += fr * total + o0 + fx;
     auto flush = [&]() {
         __syncwarp(lanes);
-        if (tile + fx * (SW + 1) + row < put) {  // the entry is held (put = tile + held * (SW + 1) + row)
+        if (tile + fx * (kWidth + 1) + row < put) {  // the entry is held (put = tile + held * (kWidth + 1) + row)
             const int c = *fcol + row0;
-            const T *from = tile + fx * (SW + 1);
+            const T *from = tile + fx * (kWidth + 1);
             int at = 0;
 #pragma unroll
-            for (int r = fr; r < SW; r += SW / kGroupFlush, at += SW / kGroupFlush * total) {
+            for (int r = fr; r < kWidth; r += SW / kGroupFlush, at += SW / kGroupFlush * total) {
                 if (r < n) {
                     pc[at] = c + r;
                     pv[at] = from[r];
@@ -276,38 +339,55 @@ __device__ __forceinline__ void group_fold(GroupSmem<T> &s, int total, int n, in
         pc += kGroupFlush;
         pv += kGroupFlush;
     };
-    typename AccT::S acc = AccT::zero();
-    auto product = [&](unsigned x, T av, T bv) {
-        acc = AccT::step(acc, av, bv);
+    // a product's operands: of the lane's row, or of its two
+    using Operand = std::conditional_t<kPair, unsigned long long, T>;
+    std::conditional_t<kPair, AccPair, typename AccT::S> acc{};
+    auto load = [&](unsigned x, Operand &av, Operand &bv) {
+        if constexpr (kPair) {
+            av = reinterpret_cast<const unsigned long long *>(a)[x & 31u];
+            bv = AccPair::pack(b[x >> 6], b1[x >> 6]);
+        } else {
+            av = a[x & 31u];
+            bv = b[x >> 6];
+        }
+    };
+    auto product = [&](unsigned x, Operand av, Operand bv) {
+        if constexpr (kPair) acc.step(av, bv);
+        else acc = AccT::step(acc, av, bv);
         if (x & 32u) {
-            *put = AccT::fin(acc);
-            acc = AccT::zero();
-            put += SW + 1;
-            if (put == tile + row + kGroupFlush * (SW + 1)) flush();
+            if constexpr (kPair) {
+                const float2 v = acc.fin();
+                put[0] = v.x;
+                put[SW] = v.y;
+            } else {
+                *put = AccT::fin(acc);
+            }
+            acc = {};
+            put += kWidth + 1;
+            if (put == tile + row + kGroupFlush * (kWidth + 1)) flush();
         }
     };
     for (; e + 4 <= e_end; e += 4) {
         unsigned x[4];
-        T av[4], bv[4];
+        Operand av[4], bv[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) x[u] = s.sched[e + u];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            av[u] = a[x[u] & 31u];
-            bv[u] = b[x[u] >> 6];
-        }
+        for (int u = 0; u < 4; ++u) load(x[u], av[u], bv[u]);
 #pragma unroll
         for (int u = 0; u < 4; ++u) product(x[u], av[u], bv[u]);
     }
     for (; e < e_end; ++e) {
         const unsigned x = s.sched[e];
-        product(x, a[x & 31u], b[x >> 6]);
+        Operand av, bv;
+        load(x, av, bv);
+        product(x, av, bv);
     }
     if (put != tile + row) flush();
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kGroupThreads, group_ctas<T>()) k_group_rows(SpgemmArgs<T> g, const int2 *__restrict__ groups,
+__global__ void __launch_bounds__(kGroupThreads, kGroupCtas) k_group_rows(SpgemmArgs<T> g, const int2 *__restrict__ groups,
                                                                  int *cursor)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -348,7 +428,14 @@ __global__ void __launch_bounds__(kGroupThreads, group_ctas<T>()) k_group_rows(S
         const bool packed = (longest & 1) && __all_sync(kFull, lane >= len_a || bl == longest);
         const int pb = longest | 1;
         const int p = __popc(heads & (lanemask_lt() | (1u << lane))) - 1;  // pencils before and with this entry, less 1
-        int base = (lane + p * (kGroupLanes - 1)) * pb;
+        // rows walked together: two per lane where there are more than 32 and their values fit
+        constexpr int kRows = GroupSmem<T>::kRows;
+        const bool wide = kRows > kGroupLanes && gr.y > kGroupLanes &&
+                          (len_a + pencils * (kRows - 1)) * pb + 8 * pencils <= GroupSmem<T>::kStage;
+        auto rows_at = [&](int rest) {  // 17 to 24 rows as 16 and the rest: three quarters of the work of 32
+            return rest > 24 ? min(wide ? kRows : kGroupLanes, rest) : min(16, rest);
+        };
+        int base = (lane + p * ((wide ? kRows : kGroupLanes) - 1)) * pb;
         if (packed) {  // as many values into 16 bytes as the pencil's first value lies in memory
             const int h = 31 - __clz(heads & (lanemask_lt() | (1u << lane)));  // the pencil's first entry
             const int first = __shfl_sync(kFull, b0, h);
@@ -379,9 +466,11 @@ __global__ void __launch_bounds__(kGroupThreads, group_ctas<T>()) k_group_rows(S
         const int products = min(s.e_start[len_a], kEsc1FlopMax);
         // A's and B's values of rows [r0, r0 + n) of the group
         auto stage = [&](int r0, int n) {
-            for (int i = warp; i < n; i += NW)
-                if (lane < len_a)
-                    copy_async(s.a + i * pa + lane, g.aval + a0 + (long long)(r0 + i) * len_a + lane);
+            for (int i = warp; i < n; i += NW) {
+                T *to = s.a + i * pa + lane;
+                if (n > kGroupLanes) to = s.a + 2 * ((i % kGroupLanes) * pa + lane) + i / kGroupLanes;
+                if (lane < len_a) copy_async(to, g.aval + a0 + (long long)(r0 + i) * len_a + lane);
+            }
             // a pencil by one warp, or by as many as there are to a pencil
             const int parts = max(1, NW / pencils);
             for (int w = warp; w < pencils * parts; w += NW) {
@@ -407,7 +496,7 @@ __global__ void __launch_bounds__(kGroupThreads, group_ctas<T>()) k_group_rows(S
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        stage(0, gr.y > 24 ? min(kGroupLanes, gr.y) : min(16, gr.y));
+        stage(0, rows_at(gr.y));
         // the pattern: products' columns, entries and positions
         unsigned col[PER], idx[PER];
         int own[PER], at[PER];
@@ -481,18 +570,19 @@ __global__ void __launch_bounds__(kGroupThreads, group_ctas<T>()) k_group_rows(S
         if (t == 0 && !fits) atomicOr(&g.info->flags, kErrCountMismatch);
         int n = 0;
         for (int r0 = 0; r0 < gr.y; r0 += n) {
-            // 17 to 24 rows as 16 and the rest: three quarters of the FMAs of a 32-row walk
-            const int rest = gr.y - r0;
-            n = rest > 24 ? min(kGroupLanes, rest) : min(16, rest);
+            n = rows_at(gr.y - r0);
             if (r0 > 0) stage(r0, n);
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             if (fits) {
                 int *pc = g.c_col + off + r0 * total;
                 T *pv = g.c_val + off + r0 * total;
-                if (n > 16) group_fold<32, T>(s, total, n, r0, pa, pb, pc, pv);
-                else if (n > 8) group_fold<16, T>(s, total, n, r0, pa, pb, pc, pv);
-                else group_fold<8, T>(s, total, n, r0, pa, pb, pc, pv);
+                if constexpr (kRows > kGroupLanes) {
+                    if (n > kGroupLanes) group_fold<32, true, T>(s, total, n, r0, pa, pb, pc, pv);
+                }
+                if (n <= 8) group_fold<8, false, T>(s, total, n, r0, pa, pb, pc, pv);
+                else if (n <= 16) group_fold<16, false, T>(s, total, n, r0, pa, pb, pc, pv);
+                else if (n <= kGroupLanes) group_fold<32, false, T>(s, total, n, r0, pa, pb, pc, pv);
             }
             __syncthreads();  // the staged values are done with
         }

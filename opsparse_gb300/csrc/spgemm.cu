@@ -429,7 +429,7 @@ int launch_groups(ops_handle_s *h, const SpgemmArgs<T> &g, int rows, cudaStream_
 {
     const int most = rows / kGroupMin + 1;
     if constexpr (kNum) {
-        k_group_rows<T><<<std::min(most, h->num_sms * group_ctas<T>()), kGroupThreads, sizeof(GroupSmem<T>), s>>>(
+        k_group_rows<T><<<std::min(most, h->num_sms * kGroupCtas), kGroupThreads, sizeof(GroupSmem<T>), s>>>(
             g, h->groups, &h->info->next_num.group);
     } else {
         SpgemmArgs<double> gc{};

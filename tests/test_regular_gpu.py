@@ -22,6 +22,8 @@ BANDS = {
     "short": ([3, 4, 9, 20, 21, 22, 40, 41, 77], list(range(16, 64, 3))),  # 144 products, B rows of 16
     # runs of B rows that start at every offset of 16 bytes, rows of 17
     "odd_pencils": ([0, 1, 2, 30, 31, 32, 63, 64, 65], list(range(0, 34, 2))),
+    # 16 runs of one B row each: staged for 32 rows together, not for 64
+    "single_rows": (list(range(0, 48, 3)), list(range(0, 51, 3))),
     "pencils": (list(range(0, 96, 3)), list(range(0, 62, 2))),  # 992 products, 32 B rows apart: not staged
 }
 
@@ -48,6 +50,7 @@ def banded(name, rows, cuts, seed):
 @pytest.mark.parametrize("name,rows,cuts,groups", [("stencil25", 25000, 0, True), ("stencil25", 30000, 350, True),
                                                    ("one_pencil", 25001, 300, True), ("short", 60000, 1000, True),
                                                    ("odd_pencils", 30001, 40, True), ("odd_pencils", 33003, 600, True),
+                                                   ("single_rows", 25003, 200, True),
                                                    ("pencils", 25000, 20, False), ("short", 1000, 10, False),
                                                    ("short", 40000, 6000, False)])
 @pytest.mark.parametrize("dtype", ["f64", "f32"])
