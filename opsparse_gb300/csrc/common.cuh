@@ -132,7 +132,7 @@ struct DevInfo {
     int groups;                   // groups of rows of one pattern (regular.cuh)
     unsigned long long d_len_a;   // A entries of the D rows
     unsigned long long d_flop;    // products of the D rows
-    int d_cursor;                 // long runs listed by the D-row short-run fold
+    int d_cursor;                 // long runs or chains listed by a short fold (D rows, backward)
     int rank_rows[3];             // E1 rows of the 1,024-product shape where B has at most 65,536
                                   // columns, by products in repeated columns: [0, 1..128, more]
 };

@@ -7,10 +7,12 @@
 //   2. read back class sizes and max products                   (host sync #1)
 //   3. symbolic kernels, one stream per non-empty class, joined back onto the caller's
 //      stream with events                                       (multi-stream bin dispatch)
-//   4. exclusive scan of row nnz into C.row_ptr (CUB)
+//   4. exclusive scan of row nnz into C.row_ptr (one CTA for few rows, else CUB)
 //   5. read back nnz(C)                                         (host sync #2)
 //   6. C allocated from the handle's stream-ordered pool
 //   7. numeric kernels on the same per-class streams, reusing step 1's classes
+// Small problems take one kernel per phase instead of step 3's and 7's classes (small_problem);
+// rows on structured grids are grouped by pattern between steps 2 and 3 (form_groups).
 // Workspace (class lists, counters, scan scratch, dense-row scratch) lives in a
 // cudaMemPool owned by the handle and is reused across calls; streams and events are
 // created once per handle, never per call.

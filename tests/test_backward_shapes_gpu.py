@@ -50,3 +50,39 @@ def test_chain_lengths(cuda, budget, need):
         if asked:
             assert np.array_equal(got.cpu().numpy().view(np.uint64), want.view(np.uint64))
     h.close()
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("budget", [None, 0], ids=["map", "search"])
+def test_rows_in_blocks(cuda, budget, dtype):
+    """C of more than 8,388,608 entries: dB walks A's rows in blocks, its folds' states kept in
+    between (FP64 bit for bit; FP32 within 1e-5 of the FP64 oracle on the same inputs, the
+    tolerance of every FP32 gradient)."""
+    rng = np.random.default_rng(23)
+    m, k, n, da_, db_ = 4000, 5000, 4000, 40, 140
+
+    def random(rows, cols, deg):
+        rpt = np.arange(rows + 1, dtype=np.int32) * deg
+        col = np.concatenate([np.sort(rng.choice(cols, deg, replace=False)) for _ in range(rows)]).astype(np.int32)
+        return rpt, col, rng.standard_normal(rows * deg).astype(np.float32).astype(np.float64)
+
+    a, b = random(m, k, da_), random(k, n, db_)
+    tdt = cuda.float64 if dtype == "f64" else cuda.float32
+    h = ops.Handle()
+    if budget is not None:
+        ops.capi.check(h.lib.ops_handle_set_map_budget(h.h, budget))
+    A, B = ops.csr_to_device(*a, m, k, dtype=tdt), ops.csr_to_device(*b, k, n, dtype=tdt)
+    op = FixedPatternSpGEMM(A, B, h)
+    assert op.nnz > 8 << 20
+    op.forward_values(A.val, B.val)
+    w = rng.standard_normal(op.nnz).astype(np.float32).astype(np.float64)
+    for _ in range(2):
+        da, db = op.backward_values(A.val, B.val, cuda.as_tensor(w).to(tdt).cuda())
+    oda, odb = oracle.backward(*a, *b, n, op.c_rpt.cpu().numpy().astype(np.int64), op.c_col.cpu().numpy(), w)
+    for got, want in ((da, oda), (db, odb)):
+        got = got.cpu().numpy()
+        if dtype == "f64":
+            assert np.array_equal(got.view(np.uint64), want.view(np.uint64))
+        else:
+            assert np.max(np.abs(got - want) / np.maximum(np.abs(want), 1.0)) <= 1e-5
+    h.close()
