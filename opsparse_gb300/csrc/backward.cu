@@ -43,9 +43,10 @@ constexpr int kGradShortMax = 64;  // chains longer than this are folded by a wa
 // dB walks A's rows in blocks of at most kGradBlock entries of C (112 MB in FP64, within
 // L2), where the columns of A are long enough for a block to hold kGradBlockMean of their
 // entries on average.  Graph of 200,000 nodes times its transpose (40 million entries): the
-// gradient kernel 557 us in one block, 470 in five, 391 in three, the step 3.21 -> 3.00 ms
-// with half the operands loaded ahead (a block's part of a column is short); uniform 100,000
-// x 60,000 x 100,000 FP32, the step 1.18 -> 0.80 ms with what a thread per entry gives.
+// gradient kernel 557 us in one block, 470 in five, 391 in three, 375 in three with half the
+// operands loaded ahead (a block's part of a column is short), the step 3.21 -> 3.00 ms;
+// uniform 100,000 x 60,000 x 100,000 FP32, the step 1.18 -> 0.80 ms with what a thread per
+// entry gives.
 constexpr int kGradBlock = 14 << 20;
 constexpr int kGradBlocksMax = 8;
 constexpr int kGradBlockMean = 2;
@@ -188,7 +189,9 @@ __device__ __forceinline__ int prod_pos(const int *__restrict__ pmap, long long 
 
 // dA, chains of at most kGradShortMax terms: one thread per A entry p = (i, j), folding
 // B row j in order, kGradBatch terms' operands loaded ahead of their FMAs.  Longer chains
-// are listed for k_grad_a_long.
+// are listed for k_grad_a_long.  (A warp that walks 32 entries' products together, through
+// shared memory, reads positions and values in order but took 438 us against 258 on a
+// graph of 200,000 nodes times its transpose; four terms ahead instead of eight, 253.)
 template <typename T, bool kMap>
 __global__ void __launch_bounds__(256) k_grad_a_short(const int *__restrict__ acol, long long nnz_a,
                                                        const int *__restrict__ arow, const int *__restrict__ brpt,
