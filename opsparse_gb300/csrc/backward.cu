@@ -324,7 +324,12 @@ __global__ void __launch_bounds__(256) k_grad_b_short(long long nnz_b, const int
             e1 = __ldg(e_hi + j);
             if (e0 == e1 && !first && !last) continue;
         }
-        const int t = (int)(q - __ldg(brpt + j));
+        const int b0 = __ldg(brpt + j);
+        const int t = (int)(q - b0);
+        if (t < 0 || t >= __ldg(brpt + j + 1) - b0) {  // not the pattern of the plan
+            atomicOr(flags, kErrCountMismatch);
+            continue;
+        }
         const int key = kMap ? 0 : __ldg(bcol + q);
         typename AccT::S s = AccT::zero();
         if constexpr (kBlocked)
@@ -377,7 +382,7 @@ __global__ void __launch_bounds__(256) k_grad_b_long(const int *__restrict__ lis
         const int b0 = __ldg(brpt + j), b1 = __ldg(brpt + j + 1);
         const int e0 = __ldg(at_ptr + j), e1 = __ldg(at_ptr + j + 1);
         const int q = qb + lane;
-        const bool qv = q < b1;
+        const bool qv = q >= b0 && q < b1;
         const int key = (!kMap && qv) ? __ldg(bcol + q) : 0;
         typename AccT::S s = AccT::zero();
         for (int eb = e0; eb < e1; eb += 32) {
@@ -430,9 +435,9 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
         OPS_CUDA(h, cudaFreeAsync(pl.mem, st));
         pl.mem = nullptr;
     }
-    if (pl.state) {
-        OPS_CUDA(h, cudaFreeAsync(pl.state, st));
-        pl.state = nullptr;
+    if (pl.at_blk) {
+        OPS_CUDA(h, cudaFreeAsync(pl.at_blk, st));
+        pl.at_blk = nullptr;
     }
     pl.valid = false;
     const int sms = h->num_sms;
@@ -518,18 +523,15 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
     // blocks of rows for dB's gathers
     pl.blocks = (int)std::min<long long>(std::min<long long>(((long long)c_nnz + kGradBlock - 1) / kGradBlock, kGradBlocksMax),
                                          nnz_a / ((long long)std::max(K, 1) * kGradBlockMean));
-    pl.at_blk = nullptr;
-    pl.state = nullptr;
     if (pl.blocks > 1 && nnz_b > 0) {
-        const size_t blk_bytes = align_up(4 * (size_t)K, 256) * (size_t)(pl.blocks - 1);
+        const size_t pitch = align_up(4 * (size_t)K, 256);
         void *bp = nullptr;
-        if (cudaMallocFromPoolAsync(&bp, align_up(8 * nb, 256) + blk_bytes, h->pool, st) == cudaSuccess) {
-            pl.state = bp;
-            pl.at_blk = reinterpret_cast<int *>(static_cast<unsigned char *>(bp) + align_up(8 * nb, 256));
+        if (cudaMallocFromPoolAsync(&bp, pitch * (size_t)(pl.blocks - 1), h->pool, st) == cudaSuccess) {
+            pl.at_blk = static_cast<int *>(bp);
             for (int b = 1; b < pl.blocks; ++b)
                 k_column_block<<<grid_of(K, 256, sms * 8), 256, 0, st>>>(
                     K, pl.at_ptr, pl.at_ent, pl.arow, c_rpt, M, (int)((long long)c_nnz * b / pl.blocks),
-                    pl.at_blk + (b - 1) * (align_up(4 * (size_t)K, 256) / 4));
+                    pl.at_blk + (b - 1) * (pitch / 4));
             OPS_CUDA(h, cudaGetLastError());
         } else {
             (void)cudaGetLastError();  // no room: one block
@@ -559,6 +561,7 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
         OPS_CUDA(h, cudaGetLastError());
     }
     OPS_CUDA(h, cudaFreeAsync(tp, st));
+    OPS_CUDA(h, cudaStreamSynchronize(st));  // the next call may use the plan from another stream
     pl.M = M;
     pl.K = K;
     pl.N = N;
@@ -608,16 +611,27 @@ int run_backward(ops_handle_s *h, int M, int K, const int *a_rpt, const int *a_c
     }
     if (db && pl.nnz_b > 0) {
         const int g1 = grid_of(pl.nnz_b, 256, sms * 16), g2 = grid_of(pl.long_b_count, 8, sms * 8);
+        // dB's folds between blocks belong to the call (calls may overlap on several streams);
+        // a captured call walks one block, as its graph would keep them
+        int blocks = pl.blocks;
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        OPS_CUDA(h, cudaStreamIsCapturing(st, &capture));
+        if (capture != cudaStreamCaptureStatusNone) blocks = 1;
+        typename Acc<T>::S *state = nullptr;
+        if (blocks > 1 && cudaMallocFromPoolAsync(reinterpret_cast<void **>(&state), sizeof(*state) * pl.nnz_b,
+                                                  h->pool, st) != cudaSuccess) {
+            (void)cudaGetLastError();  // no room: one block
+            blocks = 1;
+        }
         auto launch = [&](auto map) {
             constexpr bool kMap = decltype(map)::value;
-            auto *state = static_cast<typename Acc<T>::S *>(pl.state);
-            if (pl.blocks <= 1)
+            if (blocks <= 1)
                 k_grad_b_short<T, kMap, false><<<g1, 256, 0, st>>>(pl.nnz_b, pl.brow, b_rpt, b_col, a_val, pl.at_ptr,
                                                                    pl.at_ent, pl.at_src, c_rpt, c_col, dc, pl.pmap, db,
                                                                    flags, nullptr, nullptr, state, true, true);
-            for (int b = 0; b < pl.blocks && pl.blocks > 1; ++b) {
+            for (int b = 0; b < blocks && blocks > 1; ++b) {
                 const size_t pitch = align_up(4 * (size_t)K, 256) / 4;
-                const bool first = b == 0, last = b == pl.blocks - 1;
+                const bool first = b == 0, last = b == blocks - 1;
                 k_grad_b_short<T, kMap, true><<<g1, 256, 0, st>>>(
                     pl.nnz_b, pl.brow, b_rpt, b_col, a_val, pl.at_ptr, pl.at_ent, pl.at_src, c_rpt, c_col, dc, pl.pmap,
                     db, flags, first ? pl.at_ptr : pl.at_blk + (b - 1) * pitch,
@@ -630,7 +644,9 @@ int run_backward(ops_handle_s *h, int M, int K, const int *a_rpt, const int *a_c
         };
         if (pl.with_map) launch(std::true_type{});
         else launch(std::false_type{});
-        OPS_CUDA(h, cudaGetLastError());
+        const cudaError_t launched = cudaGetLastError();
+        if (blocks > 1) OPS_CUDA(h, cudaFreeAsync(state, st));
+        OPS_CUDA(h, launched);
     }
     return OPS_OK;
 }

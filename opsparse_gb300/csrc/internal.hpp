@@ -34,7 +34,6 @@ struct BackwardPlan {
     int long_b_count = 0;
     int blocks = 1;                 // blocks of A's rows dB is walked in
     int *at_blk = nullptr;          // [blocks - 1][K] where the later blocks start in A's columns
-    void *state = nullptr;          // [nnz_b] dB's folds between blocks
 };
 
 struct ops_handle_s {
