@@ -113,11 +113,15 @@ static __global__ void __launch_bounds__(256) k_row_links(const int *__restrict_
 }
 
 // Cuts the runs of links into groups (first row, rows) and marks their rows.  A warp takes
-// kGroupWindow rows; runs end at its window.
+// kGroupWindow rows; runs end at its window.  soff (one-pass calls, else null): the products
+// each row stages; a grouped row stages none, whatever its span, and leaves the totals.
 static __global__ void __launch_bounds__(128) k_form_groups(int M, unsigned char *__restrict__ link,
-                                                            int2 *__restrict__ groups, DevInfo *info)
+                                                            int2 *__restrict__ groups, int *__restrict__ soff,
+                                                            DevInfo *info)
 {
     const int lane = lane_id();
+    unsigned long long products = 0;  // that the lane's grouped rows would have staged
+    int rows = 0;                     // of those rows
     const int w0 = ((blockIdx.x * 128 + threadIdx.x) >> 5) * kGroupWindow;
     if (w0 >= M) return;
     unsigned mine = 0u;  // lane i: links of rows w0 + 32 i .. + 31
@@ -154,9 +158,24 @@ static __global__ void __launch_bounds__(128) k_form_groups(int M, unsigned char
             if (lane == 0) base = atomicAdd(&info->groups, n);
             base = __shfl_sync(kFull, base, 0);
             if (lane < n) groups[base + lane] = make_int2(w0 + s + kGroupRows * lane, min(kGroupRows, grouped - kGroupRows * lane));
-            for (int i = lane; i < grouped; i += 32) link[w0 + s + i] |= kGrouped;
+            for (int i = lane; i < grouped; i += 32) {
+                const int r = w0 + s + i;
+                link[r] |= kGrouped;
+                if (soff && soff[r] > 0) {
+                    products += (unsigned long long)soff[r];
+                    ++rows;
+                    soff[r] = 0;
+                }
+            }
         }
         at = e + 1;
+    }
+    if (!soff) return;
+    products = warp_sum_u64(products);
+    rows = (int)__reduce_add_sync(kFull, (unsigned)rows);
+    if (lane == 0 && rows > 0) {
+        atomicAdd(&info->staged_flop, 0ull - products);
+        atomicSub(&info->e1_one, rows);
     }
 }
 

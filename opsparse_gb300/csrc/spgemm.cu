@@ -351,8 +351,12 @@ constexpr int kMinChainRows = 20480;
 constexpr int kMinChainRun = 14;
 
 // Groups of rows of one pattern (regular.cuh), where k_setup found enough E1 rows that A's
-// next row repeats: links from B, groups, and the E1 rows outside them (h->regular).
-int form_groups(ops_handle_s *h, const DevInfo &hi, const Mat &A, const Mat &B, cudaStream_t st)
+// next row repeats: links from B, groups, and the E1 rows outside them (h->regular).  In a
+// call that may stage (want_stage), hi's staged rows and products are those outside the groups
+// afterwards: rows of a wider span than the column window would have been staged, and their
+// number decides whether the E1 class still has a numeric phase.  They are read back where
+// there may be any (one round trip, about 10 us of calls of a millisecond and more).
+int form_groups(ops_handle_s *h, DevInfo &hi, const Mat &A, const Mat &B, bool want_stage, cudaStream_t st)
 {
     h->regular = false;
     if (hi.e1_chain < kMinChainRows || hi.e1_chain < kMinChainRun * hi.e1_runs) return OPS_OK;
@@ -369,10 +373,17 @@ int form_groups(ops_handle_s *h, const DevInfo &hi, const Mat &A, const Mat &B, 
     const int sms = h->num_sms;
     k_shift_links<<<grid_for(K, 32, sms * 16), 256, 0, st>>>(B.rpt, B.col, K, B.cols, h->b_link);
     k_row_links<<<grid_for(M, 32, sms * 16), 256, 0, st>>>(A.rpt, A.col, B.rpt, M, h->b_link, h->link);
-    k_form_groups<<<(M + 4 * kGroupWindow - 1) / (4 * kGroupWindow), 128, 0, st>>>(M, h->link, h->groups, h->info);
+    k_form_groups<<<(M + 4 * kGroupWindow - 1) / (4 * kGroupWindow), 128, 0, st>>>(
+        M, h->link, h->groups, want_stage ? h->soff : nullptr, h->info);
     OPS_CUDA(h, cudaGetLastError());
     h->launches += 3;
     h->regular = true;
+    if (want_stage && hi.e1_one > 0) {
+        OPS_CUDA(h, cudaMemcpyAsync(h->h_info, h->info, sizeof(DevInfo), cudaMemcpyDeviceToHost, st));
+        OPS_CUDA(h, cudaStreamSynchronize(st));
+        hi.staged_flop = h->h_info->staged_flop;
+        hi.e1_one = h->h_info->e1_one;
+    }
     return OPS_OK;
 }
 
@@ -778,7 +789,7 @@ int run_symbolic(ops_handle_s *h, const Mat &A, const Mat &B, int *c_rpt, long l
         h->plan_valid = true;
         return OPS_OK;
     }
-    OPS_CHECK(form_groups(h, hi, A, B, st));
+    OPS_CHECK(form_groups(h, hi, A, B, want_stage, st));
     if (want_stage) OPS_CHECK(prepare_stage(h, hi, M, st));
     OPS_CHECK((launch_classes<false, double>(h, g, st)));
     if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[3], st));
