@@ -28,8 +28,8 @@ enum RowClass : int {
 
 // Extra device lists after the kNumClasses class lists: the numeric re-binning of the E1
 // rows and the size split of the E2 rows.
-// The last four split the E1 rows of a one-pass call into those computed in the counting
-// phase, by rank shape, and those left to two passes.
+// The kXlE1One lists and kXlE1Two split the E1 rows of a one-pass call into those computed in
+// the counting phase, by rank shape, and those left to two passes.
 enum : int {
     kXlE1Small = 0,     // numeric re-binning of the E1 rows (PickE1)
     kXlE1Hash = 1,
@@ -41,7 +41,8 @@ enum : int {
     kXlE1Two = 7,
     kXlE1OneLarge = 8,
     kXlE1OneHalf = 9,
-    kNumExtraLists = 10
+    kXlE1Rest = 10,     // E1 rows outside the groups of one pattern (regular.cuh)
+    kNumExtraLists = 11
 };
 constexpr int kNumLists = kNumClasses + kNumExtraLists;
 
@@ -130,6 +131,7 @@ struct DevInfo {
     int e1_chain;                 // E1 rows whose A row the next row of A repeats, moved by one column
     int e1_runs;                  // runs of such rows, cut at every 32 rows
     int groups;                   // groups of rows of one pattern (regular.cuh)
+    int e1_rest;                  // E1 rows outside them
     unsigned long long d_len_a;   // A entries of the D rows
     unsigned long long d_flop;    // products of the D rows
     int d_cursor;                 // long runs or chains listed by a short fold (D rows, backward)

@@ -73,10 +73,8 @@ struct PickStaged {
     const int *soff;
     const int *row_flop;
     const int *arpt;
-    const unsigned char *link;  // rows in groups are dropped (null: there are none)
     __device__ int operator()(int r) const
     {
-        if (link && (link[r] & kGrouped)) return -1;
         if (soff[r + 1] <= soff[r]) return 1;
         const int shape = e1_shape(row_flop[r], arpt[r + 1] - arpt[r]);
         return shape == 0 ? 0 : (shape == 1 ? 3 : 2);

@@ -228,7 +228,7 @@ T *stage_vals(ops_handle_s *h)
 // to the staging area at soff[r] and their counts to c_rpt, in place of the counting
 // kernels.  The E1 rows it does not stage are counted as usual.
 template <typename T, typename GA>
-int launch_staged_class(ops_handle_s *h, const GA &gs, int c, const int *list, int n, cudaStream_t s)
+int launch_staged_class(ops_handle_s *h, const GA &gs, int c, const int *list, const int *count, int n, cudaStream_t s)
 {
     SpgemmArgs<T> g{};
     g.arpt = gs.arpt;
@@ -267,7 +267,7 @@ int launch_staged_class(ops_handle_s *h, const GA &gs, int c, const int *list, i
             int *one_large = xl + kXlE1OneLarge * M;
             int *one_half = xl + kXlE1OneHalf * M;
             k_split_list<4, PickStaged><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
-                list, &h->info->counts[c], PickStaged{h->soff, g.row_flop, g.arpt, h->regular ? h->link : nullptr}, one, (int)M, h->info->split1);
+                list, count, PickStaged{h->soff, g.row_flop, g.arpt}, one, (int)M, h->info->split1);
             OPS_CUDA(h, cudaGetLastError());
             ++h->launches;
             OPS_CUDA(h, cudaEventRecord(h->ev_x_fork[0], s));
@@ -515,12 +515,24 @@ int launch_classes(ops_handle_s *h, const SpgemmArgs<T> &g, cudaStream_t st)
             ++h->launches;
         }
         if (h->timing >= 2) OPS_CUDA(h, cudaEventRecord(h->ev_k[kNum][c][0], s));
-        if (c == kClsE1 && h->regular && !(kNum && h->no_groups)) {  // the groups of one pattern, then the other rows
-            OPS_CHECK((launch_groups<kNum, T>(h, g, n, s)));
+        const int *count = &h->info->counts[c];
+        if (c == kClsE1 && h->regular) {
+            // the groups of one pattern, then the other rows: a list of their own, made while
+            // counting and kept for every numeric phase of the plan, whatever was staged
+            if (!(kNum && h->no_groups)) OPS_CHECK((launch_groups<kNum, T>(h, g, n, s)));
+            int *rest = xl + kXlE1Rest * M;
+            if (!kNum) {
+                k_split_list<1, PickUngrouped><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
+                    list, count, PickUngrouped{h->link}, rest, (int)M, &h->info->e1_rest);
+                OPS_CUDA(h, cudaGetLastError());
+                ++h->launches;
+            }
+            list = rest;
+            count = &h->info->e1_rest;
         }
         if (staged && !kNum) {  // one-pass call: numeric into the staging area
-            OPS_CHECK(h->op_dtype == OPS_F64 ? launch_staged_class<double>(h, g, c, list, n, s)
-                                             : launch_staged_class<float>(h, g, c, list, n, s));
+            OPS_CHECK(h->op_dtype == OPS_F64 ? launch_staged_class<double>(h, g, c, list, count, n, s)
+                                             : launch_staged_class<float>(h, g, c, list, count, n, s));
         } else
         switch (c) {
             case kClsR8:  // numeric only: walks the rows in order
@@ -537,19 +549,9 @@ int launch_classes(ops_handle_s *h, const SpgemmArgs<T> &g, cudaStream_t st)
                 break;
             case kClsE1: {
                 if (!kNum) {  // distinct-column count: one warp per row, table of 2*flop slots
-                    if (h->regular) {
-                        int *two = xl + kXlE1Two * M;
-                        k_split_list<1, PickUngrouped><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
-                            list, &h->info->counts[c], PickUngrouped{h->link}, two, (int)M, &h->info->split1[1]);
-                        k_warp_rows<false, T, 2 * kEsc1FlopMax>
-                            <<<grid_for(n, kWarpRowsThreads / 32, sms * 3), kWarpRowsThreads,
-                               warp_rows_smem<false, T, 2 * kEsc1FlopMax>(), s>>>(g, two, &h->info->split1[1]);
-                        h->launches += 1;
-                        break;
-                    }
                     k_warp_rows<false, T, 2 * kEsc1FlopMax>
                         <<<grid_for(n, kWarpRowsThreads / 32, sms * 3), kWarpRowsThreads,
-                           warp_rows_smem<false, T, 2 * kEsc1FlopMax>(), s>>>(g, list, &h->info->counts[c]);
+                           warp_rows_smem<false, T, 2 * kEsc1FlopMax>(), s>>>(g, list, count);
                     break;
                 }
                 // re-bin by output size: the warp's rank shape and warp hash on this stream,
@@ -559,9 +561,8 @@ int launch_classes(ops_handle_s *h, const SpgemmArgs<T> &g, cudaStream_t st)
                 int *half_list = xl + kXlE1Half * M;
                 int *hash_list = xl + kXlE1Hash * M;
                 int *rank_list = xl + kXlE1Rank * M;
-                const bool two = staged || h->regular;
-                const int *e1_list = two ? xl + kXlE1Two * M : list;
-                const int *e1_count = two ? &h->info->split1[1] : &h->info->counts[c];
+                const int *e1_list = staged ? xl + kXlE1Two * M : list;
+                const int *e1_count = staged ? &h->info->split1[1] : count;
                 k_split_list<4, PickE1><<<grid_for(n, 256, sms * 4), 256, 0, s>>>(
                     e1_list, e1_count, PickE1{g.c_rpt, g.row_flop, g.arpt}, small_list, (int)M, h->info->split);
                 OPS_CUDA(h, cudaGetLastError());

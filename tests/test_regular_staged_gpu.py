@@ -1,6 +1,7 @@
 """Groups of rows of one pattern (regular.cuh) in calls that compute rows while they count:
 grouped rows whose products span more columns than the column window (32,768) would be staged
-as well, and must not be.  Grids of a wide cross-section and bands of two distant clusters,
+as well, and must not be; a numeric call with new values on the plan of such a call computes every row.
+Grids of a wide cross-section and bands of two distant clusters,
 alone, cut by rows that miss an entry, and beside narrow bands, irregular and short rows; both
 ways to call, every mode, FP64 and FP32, against the oracle bit for bit."""
 import numpy as np
@@ -92,3 +93,29 @@ def test_grouped_rows_are_not_staged(cuda, name, dtype):
             for stream in (None, other):
                 check(h.spgemm_oneshot(A, B, stream=stream).to_host(), want)
                 assert grouped_rows(h) > A.rows // 4
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("name", [n for n in CASES if n != "grid25x100x100"])
+def test_numeric_on_a_one_pass_plan(cuda, name, dtype):
+    a, b, A, B, want = on_device(cuda, name, dtype)
+    rng = np.random.default_rng(9)
+    c_rpt = cuda.as_tensor(want[0].astype(np.int32)).cuda()
+    nnz = len(want[1])
+    other = cuda.cuda.Stream()
+    for mode in (1, 2):
+        with ops.Handle() as h:
+            h.set_one_pass(mode)
+            for stream in (None, other):  # two halves; ops_spgemm
+                h.spgemm_oneshot(A, B, stream=stream)
+                new = [rng.standard_normal(len(m[1])).astype(m[2].dtype) for m in (a, b)]
+                if B is A:
+                    new[1] = new[0]
+                A2, B2 = (ops.CsrMatrix(m.rows, m.cols, m.rpt, m.col, cuda.as_tensor(v).cuda())
+                          for m, v in zip((A, B), new))
+                expect = oracle.spgemm(a[0], a[1], new[0], b[0], b[1], new[1], B.cols, dtype=a[2].dtype)
+                for _ in range(2):
+                    c_col = cuda.full((nnz,), -1, dtype=cuda.int32, device="cuda")
+                    c_val = cuda.full((nnz,), 7.0, dtype=A.val.dtype, device="cuda")
+                    h.numeric(A2, B2, c_rpt, nnz, c_col=c_col, c_val=c_val)
+                    check((want[0], c_col.cpu().numpy(), c_val.cpu().numpy()), expect)
