@@ -194,8 +194,9 @@ int ops_spgemm_check(ops_handle_t handle, void *stream);
  * order; dB_jk = sum_i A_ij dC_ik folded over ascending i; FP64 uses one FMA per term,
  * FP32 the Dot2 compensated sum.  The first call for a pattern builds a plan on the handle
  * (A's transpose order and, if it fits the map budget, each product's position in C);
- * later calls with the same pattern pointers reuse it.  Asynchronous; ops_spgemm_check
- * reports OPS_COUNT_MISMATCH if C's pattern lacks a product of A and B. */
+ * later calls with the same pattern pointers reuse it, also at the same time on several
+ * streams (their error flags are shared: each call clears them).  Asynchronous;
+ * ops_spgemm_check reports OPS_COUNT_MISMATCH if C's pattern lacks a product of A and B. */
 int ops_spgemm_backward(ops_handle_t handle, int dtype, int32_t rows_a, int32_t cols_a, int32_t cols_b,
                         const int32_t *a_rpt, const int32_t *a_col, const void *a_val, int64_t a_nnz,
                         const int32_t *b_rpt, const int32_t *b_col, const void *b_val, int64_t b_nnz,

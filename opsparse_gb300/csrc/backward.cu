@@ -586,33 +586,32 @@ int run_backward(ops_handle_s *h, int M, int K, const int *a_rpt, const int *a_c
     const int sms = h->num_sms;
     int *flags = &h->info->flags;
     if (da && pl.nnz_a > 0) {
-        // thread per A entry for short chains; the long ones are listed and get a warp each
+        // thread per A entry for short chains; the long ones are listed and get a warp each.
+        // The list and its length belong to the call: calls may overlap on several streams
         int *long_list = nullptr;
-        OPS_CUDA(h, cudaMallocFromPoolAsync(reinterpret_cast<void **>(&long_list), sizeof(int) * pl.nnz_a, h->pool,
-                                            st));
-        OPS_CUDA(h, cudaMemsetAsync(&h->info->d_cursor, 0, sizeof(int), st));
+        OPS_CUDA(h, cudaMallocFromPoolAsync(reinterpret_cast<void **>(&long_list), sizeof(int) * (pl.nnz_a + 1),
+                                            h->pool, st));
+        int *long_count = long_list + pl.nnz_a;
+        OPS_CUDA(h, cudaMemsetAsync(long_count, 0, sizeof(int), st));
         const int g1 = grid_of(pl.nnz_a, 256, sms * 16);
         if (pl.with_map) {
             k_grad_a_short<T, true><<<g1, 256, 0, st>>>(a_col, pl.nnz_a, pl.arow, b_rpt, b_col, b_val, c_rpt, c_col, dc,
-                                                        pl.pos_base, pl.pmap, da, long_list, &h->info->d_cursor, flags);
+                                                        pl.pos_base, pl.pmap, da, long_list, long_count, flags);
             k_grad_a_long<T, true><<<sms * 8, 256, 0, st>>>(a_col, pl.arow, b_rpt, b_col, b_val, c_rpt, c_col, dc,
-                                                            pl.pos_base, pl.pmap, da, long_list, &h->info->d_cursor,
-                                                            flags);
+                                                            pl.pos_base, pl.pmap, da, long_list, long_count, flags);
         } else {
             k_grad_a_short<T, false><<<g1, 256, 0, st>>>(a_col, pl.nnz_a, pl.arow, b_rpt, b_col, b_val, c_rpt, c_col,
-                                                         dc, pl.pos_base, pl.pmap, da, long_list, &h->info->d_cursor,
-                                                         flags);
+                                                         dc, pl.pos_base, pl.pmap, da, long_list, long_count, flags);
             k_grad_a_long<T, false><<<sms * 8, 256, 0, st>>>(a_col, pl.arow, b_rpt, b_col, b_val, c_rpt, c_col, dc,
-                                                             pl.pos_base, pl.pmap, da, long_list, &h->info->d_cursor,
-                                                             flags);
+                                                             pl.pos_base, pl.pmap, da, long_list, long_count, flags);
         }
         OPS_CUDA(h, cudaGetLastError());
         OPS_CUDA(h, cudaFreeAsync(long_list, st));
     }
     if (db && pl.nnz_b > 0) {
         const int g1 = grid_of(pl.nnz_b, 256, sms * 16), g2 = grid_of(pl.long_b_count, 8, sms * 8);
-        // dB's folds between blocks belong to the call (calls may overlap on several streams);
-        // a captured call walks one block, as its graph would keep them
+        // dB's folds between blocks belong to the call as well; a captured call walks one
+        // block, as its graph would keep them
         int blocks = pl.blocks;
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         OPS_CUDA(h, cudaStreamIsCapturing(st, &capture));

@@ -1,0 +1,91 @@
+"""Backward calls beside one another and by other routes than one call at a time: two of one
+handle at once on two streams, a captured one, and one whose B no longer has an entry of the
+plan.  FP64, bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+import oracle
+import opsparse_gb300 as ops
+from opsparse_gb300 import capi
+from opsparse_gb300.autograd import FixedPatternSpGEMM
+
+pytestmark = pytest.mark.gpu
+
+
+def regular_degrees(rows, cols, deg, rng):
+    col = np.concatenate([np.sort(rng.choice(cols, deg, replace=False)) for _ in range(rows)]).astype(np.int32)
+    return np.arange(rows + 1, dtype=np.int32) * deg, col, rng.standard_normal(rows * deg)
+
+
+class Product:
+    """A fixed product on a handle, its gradients from the library and from the oracle."""
+
+    def __init__(self, cuda, m, k, n, deg_a, deg_b, seed=31):
+        self.cuda, self.rng = cuda, np.random.default_rng(seed)
+        self.a, self.b = regular_degrees(m, k, deg_a, self.rng), regular_degrees(k, n, deg_b, self.rng)
+        self.A, self.B = ops.csr_to_device(*self.a, m, k), ops.csr_to_device(*self.b, k, n)
+        self.h = ops.Handle()
+        self.op = FixedPatternSpGEMM(self.A, self.B, self.h)
+        self.op.forward_values(self.A.val, self.B.val)  # fills C's columns
+
+    def dc(self):
+        return self.cuda.as_tensor(self.rng.standard_normal(self.op.nnz)).cuda()
+
+    def outputs(self):
+        return self.cuda.full_like(self.A.val, np.nan), self.cuda.full_like(self.B.val, np.nan)
+
+    def call(self, dc, da, db, stream):
+        A, B, op = self.A, self.B, self.op
+        capi.check(self.h.lib.ops_spgemm_backward(
+            self.h.h, capi.OPS_F64, A.rows, A.cols, B.cols, A.rpt.data_ptr(), A.col.data_ptr(), A.val.data_ptr(), A.nnz,
+            B.rpt.data_ptr(), B.col.data_ptr(), B.val.data_ptr(), B.nnz, op.c_rpt.data_ptr(), op.c_col.data_ptr(),
+            dc.data_ptr(), da.data_ptr() if da is not None else None, db.data_ptr(), ops._stream_ptr(stream)), self.h.h)
+
+    def check(self, dc, da, db):
+        want = oracle.backward(*self.a, *self.b, self.B.cols, self.op.c_rpt.cpu().numpy().astype(np.int64),
+                               self.op.c_col.cpu().numpy(), dc.cpu().numpy())
+        for got, w in zip((da, db), want):
+            assert np.array_equal(got.cpu().numpy().view(np.uint64), w.view(np.uint64))
+
+
+@pytest.mark.parametrize("blocks", [False, True], ids=["one_block", "blocks"])
+def test_two_streams_at_once(cuda, blocks):
+    """Chains of dA longer than 64 (listed), with dB in one block and in two."""
+    p = Product(cuda, *((5000, 6000, 5000, 36, 140) if blocks else (3000, 800, 4000, 20, 90)))
+    assert (p.op.nnz > 14 << 20) == blocks
+    first, streams = p.outputs(), [cuda.cuda.Stream(), cuda.cuda.Stream()]
+    p.call(p.dc(), *first, None)  # the plan
+    cuda.cuda.synchronize()
+    dcs = [p.dc(), p.dc()]
+    rounds = [[p.outputs(), p.outputs()] for _ in range(4)]
+    cuda.cuda.synchronize()
+    for outs in rounds:
+        for i in (0, 1):
+            p.call(dcs[i], *outs[i], streams[i])
+    cuda.cuda.synchronize()
+    capi.check(p.h.lib.ops_spgemm_check(p.h.h, ops._stream_ptr()), p.h.h)
+    for i in (0, 1):
+        p.check(dcs[i], *rounds[0][i])
+        for outs in rounds[1:]:
+            assert all(bool((x == y).all()) for x, y in zip(outs[i], rounds[0][i]))
+    p.h.close()
+
+
+def test_captured_call(cuda):
+    """A built plan's call in a graph, replayed with new dC; C of more entries than one block."""
+    p = Product(cuda, 5000, 6000, 5000, 36, 140)
+    dc, (da, db) = p.dc(), p.outputs()
+    p.call(dc, da, db, None)
+    cuda.cuda.synchronize()
+    graph = cuda.cuda.CUDAGraph()
+    with cuda.cuda.graph(graph):
+        p.call(dc, da, db, cuda.cuda.current_stream())
+    for _ in range(2):
+        dc.copy_(p.dc())
+        da.fill_(np.nan)
+        db.fill_(np.nan)
+        graph.replay()
+    cuda.cuda.synchronize()
+    p.check(dc, da, db)
+    del graph
+    p.h.close()
