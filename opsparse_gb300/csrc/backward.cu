@@ -362,9 +362,9 @@ __global__ void __launch_bounds__(256) k_grad_b_short(long long nnz_b, const int
 // over the entries q, each folding the A entries of column j in ascending row order.  All
 // lanes walk the same column entries, so the warp loads 32 of them at once (one per lane) and
 // shares them by shuffle; each lane then loads kGradBatch terms' positions and dC values
-// ahead of its FMAs.
+// ahead of its FMAs.  Of the plan's entries of row j, those outside B's row are refused.
 template <typename T, bool kMap>
-__global__ void __launch_bounds__(256) k_grad_b_long(const int *__restrict__ list, int count,
+__global__ void __launch_bounds__(256) k_grad_b_long(const int *__restrict__ list, int count, long long nnz_b,
                                                       const int *__restrict__ brow, const int *__restrict__ brpt,
                                                       const int *__restrict__ bcol, const T *__restrict__ aval,
                                                       const int *__restrict__ at_ptr, const int *__restrict__ at_ent,
@@ -383,6 +383,7 @@ __global__ void __launch_bounds__(256) k_grad_b_long(const int *__restrict__ lis
         const int e0 = __ldg(at_ptr + j), e1 = __ldg(at_ptr + j + 1);
         const int q = qb + lane;
         const bool qv = q >= b0 && q < b1;
+        if (!qv && q < nnz_b && __ldg(brow + q) == j) atomicOr(flags, kErrCountMismatch);
         const int key = (!kMap && qv) ? __ldg(bcol + q) : 0;
         typename AccT::S s = AccT::zero();
         for (int eb = e0; eb < e1; eb += 32) {
@@ -637,9 +638,9 @@ int run_backward(ops_handle_s *h, int M, int K, const int *a_rpt, const int *a_c
                     last ? pl.at_ptr + 1 : pl.at_blk + b * pitch, state, first, last);
             }
             if (pl.long_b_count > 0)
-                k_grad_b_long<T, kMap><<<g2, 256, 0, st>>>(pl.long_b, pl.long_b_count, pl.brow, b_rpt, b_col, a_val,
-                                                           pl.at_ptr, pl.at_ent, pl.at_src, c_rpt, c_col, dc, pl.pmap,
-                                                           db, flags);
+                k_grad_b_long<T, kMap><<<g2, 256, 0, st>>>(pl.long_b, pl.long_b_count, pl.nnz_b, pl.brow, b_rpt, b_col,
+                                                           a_val, pl.at_ptr, pl.at_ent, pl.at_src, c_rpt, c_col, dc,
+                                                           pl.pmap, db, flags);
         };
         if (pl.with_map) launch(std::true_type{});
         else launch(std::false_type{});

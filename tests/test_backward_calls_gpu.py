@@ -89,3 +89,25 @@ def test_captured_call(cuda):
     p.check(dc, da, db)
     del graph
     p.h.close()
+
+
+@pytest.mark.parametrize("rows", [1000, 3000], ids=["short_column", "long_column"])
+def test_entry_off_the_plan_is_refused(cuda, rows):
+    """B's last row loses its last entry behind the plan's back: no gradient for it, an error.
+    Columns of A of about 25 entries (a thread per entry of B) and of about 75 (a warp)."""
+    p = Product(cuda, rows, 800, 4000, 20, 30)
+    dc, (da, db) = p.dc(), p.outputs()
+    p.call(dc, None, db, None)
+    capi.check(p.h.lib.ops_spgemm_check(p.h.h, ops._stream_ptr()), p.h.h)
+    last = float(db[-1])
+    assert np.isfinite(last)
+    p.B.rpt[-1] -= 1
+    db.fill_(np.nan)
+    p.call(dc, None, db, None)
+    assert p.h.lib.ops_spgemm_check(p.h.h, ops._stream_ptr()) == capi.OPS_COUNT_MISMATCH
+    assert bool(cuda.isnan(db[-1])) and bool(cuda.isfinite(db[:-1]).all())
+    p.B.rpt[-1] += 1  # the handle and its plan stay usable
+    p.call(dc, None, db, None)
+    capi.check(p.h.lib.ops_spgemm_check(p.h.h, ops._stream_ptr()), p.h.h)
+    assert float(db[-1]) == last
+    p.h.close()
