@@ -440,6 +440,10 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
         OPS_CUDA(h, cudaFreeAsync(pl.at_blk, st));
         pl.at_blk = nullptr;
     }
+    if (pl.pmap) {
+        OPS_CUDA(h, cudaFreeAsync(pl.pmap, st));
+        pl.pmap = nullptr;
+    }
     pl.valid = false;
     const int sms = h->num_sms;
     const size_t na = (size_t)std::max<long long>(nnz_a, 1);
@@ -540,7 +544,6 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
         }
     }
     pl.with_map = products > 0 && products <= INT_MAX && (size_t)products * 4 <= h->map_budget;
-    pl.pmap = nullptr;
     if (pl.with_map) {
         void *mp = nullptr;
         cudaError_t e = cudaMallocFromPoolAsync(&mp, (size_t)products * 4, h->pool, st);

@@ -111,3 +111,41 @@ def test_entry_off_the_plan_is_refused(cuda, rows):
     capi.check(p.h.lib.ops_spgemm_check(p.h.h, ops._stream_ptr()), p.h.h)
     assert float(db[-1]) == last
     p.h.close()
+
+
+def used(cuda):
+    cuda.cuda.synchronize()
+    free, total = cuda.cuda.mem_get_info()
+    return total - free
+
+
+def test_replaced_plans_are_given_back(cuda):
+    """Each plan of a fixed product of 16.2 million products holds a map of 65 MB; twelve more of
+    them on one handle, and on handles of their own, take no more memory than the first two did."""
+    p = Product(cuda, 6000, 800, 4000, 30, 90)
+    dc, (da, db) = p.dc(), p.outputs()
+
+    def build(h):
+        for budget in (8 << 30, 8 << 30):  # setting the budget drops the plan
+            capi.check(h.lib.ops_handle_set_map_budget(h.h, budget))
+            p.h = h
+            p.call(dc, da, db, None)
+            assert p.op.plan_info() == (16_200_000, True)
+
+    own = p.h
+    build(own)
+    before = used(cuda)
+    for _ in range(6):
+        build(own)
+    assert used(cuda) - before < 64 << 20
+    p.check(dc, da, db)
+    with ops.Handle() as h:
+        p.op.h = h
+        build(h)
+    before = used(cuda)
+    for _ in range(6):
+        with ops.Handle() as h:
+            p.op.h = h
+            build(h)
+    assert used(cuda) - before < 64 << 20
+    own.close()
