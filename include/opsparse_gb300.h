@@ -109,8 +109,8 @@ typedef struct {
                                  default 4) */
     int32_t batch_persistent; /* batches: 1 (default) = one setup kernel and one persistent
                                  kernel per row-size queue and phase over every problem's rows
-                                 (where every row has at most 4,096 products and 1,280 A
-                                 entries), 0 = per-segment pipeline */
+                                 (where every row has at most 4,096 products, and at most
+                                 1,280 of them or A entries), 0 = per-segment pipeline */
     int32_t batch_warp_max;   /* threads per row in the persistent batch kernels: rows of at most
                                  this many products (128..512, default 512) get a warp (up to
                                  256 products) or 64 threads, larger rows a 128-thread CTA (up
@@ -224,9 +224,9 @@ typedef struct ops_batch_s *ops_batch_t;
 
 /* Plans a batch: per-problem product counts, grouping into segments whose products fit
  * int32 and block-diagonal layout of each segment; then, where every row has at most
- * 4,096 products and 1,280 A entries (and ops_tuning.batch_persistent is on), one setup
- * kernel that puts every row of every problem into one of four row-size queues and one
- * persistent kernel per queue that counts them all; otherwise a row classification and
+ * 4,096 products, and at most 1,280 of them or A entries (and ops_tuning.batch_persistent is
+ * on), one setup kernel that puts every row of every problem into one of five row-size queues
+ * and one persistent kernel per queue that counts them all; otherwise a row classification and
  * symbolic phase per segment.  Then each segment's scan and the allocation of every C_b.  The items' value
  * pointers are read by ops_batch_execute, which may be called repeatedly with new values
  * in the same arrays.  The handle's row-class thresholds are used.  Synchronizes. */

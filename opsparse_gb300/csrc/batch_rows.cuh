@@ -9,7 +9,8 @@
 //   kQ512:  at most warp_max (<= 512) products (and at most 192 A entries);
 //   kQE1:   at most 1,024 products (and at most 512 A entries);
 //   kQMid:  at most 4,096 products (and at most 1,280 A entries).
-// A row joins the first that takes it.
+// A row joins the first that takes it.  The shapes hold A entries with products only, of which
+// a row has no more than products: longer rows of B rows that are mostly empty join as well.
 // Rows beyond all five are only counted; a batch that has any runs the per-segment pipeline
 // instead.  Each queue is then drained by ONE persistent kernel per phase that spans every
 // problem: its warps (or CTAs) take rows through the queue's atomic cursor until it is
@@ -90,7 +91,7 @@ static __global__ void __launch_bounds__(256) k_batch_setup(const SpgemmArgs<dou
                 }
             }
             if (bad) atomicOr(&q->flags, kErrBadColumn);
-            const int lenA = a1 - a0;
+            const int lenA = (int)min((long long)(a1 - a0), flop);  // A entries with products, at most
             const_cast<int *>(g.row_flop)[r] = flop > INT_MAX ? INT_MAX : (int)flop;
             if (flop == 0) g.c_rpt[r] = 0;
             else if (flop <= kBatchQ128) cls = kQ128;
