@@ -335,6 +335,8 @@ class Batch:
         """(rpt, col, val, nnz) of C_i as torch views of the batch's device storage (valid
         until close())."""
         torch = _torch()
+        if not 0 <= i < self.n:
+            check(capi.OPS_INVALID_ARGUMENT)
         rpt, col, val, rows, nnz = self._results()
         base, at = rpt[i]
         r = base[at:at + rows[i]]
