@@ -139,6 +139,12 @@ struct DevInfo {
                                   // columns, by products in repeated columns: [0, 1..128, more]
 };
 
+// Whether k_setup found a row that the small problems' one kernel does not take.
+__host__ __device__ inline bool beyond_small(const DevInfo &d)
+{
+    return d.counts[kClsE2] > 0 || d.counts[kClsD] > 0 || d.e1_size[1] > 0 || d.e1_size[2] > 0;
+}
+
 // Arguments shared by every SpGEMM kernel.
 template <typename T>
 struct SpgemmArgs {

@@ -441,12 +441,14 @@ static __global__ void __launch_bounds__(kSetupThreads) k_setup(const int *__res
 }
 
 // Exclusive scan in place of x[0, n) by one CTA: for row counts of small problems, where the
-// two launches of a device-wide scan cost more than its bandwidth.
+// two launches of a device-wide scan cost more than its bandwidth.  small (or null): leaves x
+// as it is where the counts are not complete, some row being beyond a small problem.
 constexpr int kScanMax = 32769;
 
-static __global__ void __launch_bounds__(1024) k_scan_rows(int *__restrict__ x, int n)
+static __global__ void __launch_bounds__(1024) k_scan_rows(int *__restrict__ x, int n, const DevInfo *small)
 {
     __shared__ int s_sums[32];
+    if (small && beyond_small(*small)) return;
     int carry = 0;
     for (int i0 = 0; i0 < n; i0 += 4096) {
         const int i = i0 + 4 * (int)threadIdx.x;

@@ -770,12 +770,13 @@ __global__ void __launch_bounds__(Sh::kThreads, Sh::kMinBlocks)
 // RankS::kAEntries A entries) by one kernel, a warp per row in row order: the classes' kernels,
 // each a launch and two events on a stream of its own, take longer to launch than to run.
 // Symbolic: the rows that k_setup left to count (not those of at most r8 products and A
-// entries).  Does nothing where k_setup found a bad column of A.
+// entries).  Does nothing where k_setup found a bad column of A or a row too large for it: the
+// usual pipeline then goes on from k_setup's classes.
 template <bool kNum, typename T>
 __global__ void __launch_bounds__(RankS::kThreads, RankS::kMinBlocks) k_rank_all(SpgemmArgs<T> g, int r8)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    if (!kNum && g.info->flags) return;
+    if (!kNum && (g.info->flags || beyond_small(*g.info))) return;
     const int warp = threadIdx.x >> 5;
     const RankSmem<RankS, T> sm(smem_raw + (size_t)warp * RankS::template group_bytes<kNum>());
     const int levels = rank_levels(g.N, RankS::kTop);

@@ -190,10 +190,11 @@ int grid_for(long long work_items, int per_block, int cap)
 }
 
 // Row pointers of C (or staging offsets) from counts, in place: x[0, M] -> exclusive prefix.
-int scan_rows(ops_handle_s *h, int *x, int M, cudaStream_t st)
+// small: the counts of a small problem, complete only if no row is beyond it.
+int scan_rows(ops_handle_s *h, int *x, int M, cudaStream_t st, bool small = false)
 {
     if (M + 1 <= kScanMax) {
-        k_scan_rows<<<1, 1024, 0, st>>>(x, M + 1);
+        k_scan_rows<<<1, 1024, 0, st>>>(x, M + 1, small ? h->info : nullptr);
         OPS_CUDA(h, cudaGetLastError());
     } else {
         size_t cb = h->cub_bytes;
@@ -729,37 +730,33 @@ int run_symbolic(ops_handle_s *h, const Mat &A, const Mat &B, int *c_rpt, long l
     g.c_rpt = c_rpt;
     g.info = h->info;
     // small problems: every row by one kernel, the scan behind it, one host sync for all of
-    // it.  It is launched before the row sizes are known, where their mean is small; if some
-    // row is too large for it, the usual pipeline starts over.
+    // it.  They are launched before the row sizes are known, where their mean is small; if some
+    // row is too large they do nothing, and the usual pipeline goes on from the classes.
+    static_assert(kSmallRows + 1 <= kScanMax, "a small problem's counts are scanned by one CTA");
     bool small = small_problem(h, A, B);
-    DevInfo hi;
-    for (;;) {
-        OPS_CUDA(h, cudaMemsetAsync(h->info, 0, sizeof(DevInfo), st));
-        if (M == 0) OPS_CUDA(h, cudaMemsetAsync(c_rpt, 0, sizeof(int), st));
-        if (M == 0 && want_stage) OPS_CUDA(h, cudaMemsetAsync(h->soff, 0, sizeof(int), st));
-        if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[1], st));
-        if (M > 0) {
-            k_setup<<<(M + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, st>>>(
-                A.rpt, A.col, B.rpt, B.col, M, A.cols, B.cols, h->row_flop, h->lists, c_rpt,
-                want_stage ? h->soff : nullptr, h->link, h->info, h->th);
-            OPS_CUDA(h, cudaGetLastError());
-            ++h->launches;
-        }
-        if (small) {
-            if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[2], st));
-            OPS_CHECK((launch_all<false, double>(h, g, st)));
-            if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[3], st));
-            OPS_CHECK(scan_rows(h, c_rpt, M, st));
-            if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[4], st));
-        }
-        OPS_CUDA(h, cudaMemcpyAsync(h->h_info, h->info, sizeof(DevInfo), cudaMemcpyDeviceToHost, st));
-        if (h->timing && !small) OPS_CUDA(h, cudaEventRecord(h->ev_t[2], st));
-        OPS_CUDA(h, cudaStreamSynchronize(st));
-        hi = *h->h_info;
-        if (!small || (hi.counts[kClsE2] == 0 && hi.counts[kClsD] == 0 && hi.e1_size[1] == 0 && hi.e1_size[2] == 0))
-            break;
-        small = false;
+    OPS_CUDA(h, cudaMemsetAsync(h->info, 0, sizeof(DevInfo), st));
+    if (M == 0) OPS_CUDA(h, cudaMemsetAsync(c_rpt, 0, sizeof(int), st));
+    if (M == 0 && want_stage) OPS_CUDA(h, cudaMemsetAsync(h->soff, 0, sizeof(int), st));
+    if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[1], st));
+    if (M > 0) {
+        k_setup<<<(M + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, st>>>(
+            A.rpt, A.col, B.rpt, B.col, M, A.cols, B.cols, h->row_flop, h->lists, c_rpt,
+            want_stage ? h->soff : nullptr, h->link, h->info, h->th);
+        OPS_CUDA(h, cudaGetLastError());
+        ++h->launches;
     }
+    if (small) {
+        if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[2], st));
+        OPS_CHECK((launch_all<false, double>(h, g, st)));
+        if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[3], st));
+        OPS_CHECK(scan_rows(h, c_rpt, M, st, true));
+        if (h->timing) OPS_CUDA(h, cudaEventRecord(h->ev_t[4], st));
+    }
+    OPS_CUDA(h, cudaMemcpyAsync(h->h_info, h->info, sizeof(DevInfo), cudaMemcpyDeviceToHost, st));
+    if (h->timing && !small) OPS_CUDA(h, cudaEventRecord(h->ev_t[2], st));
+    OPS_CUDA(h, cudaStreamSynchronize(st));
+    DevInfo hi = *h->h_info;
+    if (beyond_small(hi)) small = false;
     if (hi.flags & kErrBadColumn)
         return fail(h, OPS_INVALID_CSR, small ? "A or B has a column index outside [0, cols)"
                                               : "A has a column index outside [0, cols)");
