@@ -516,14 +516,22 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
                                                                      &h->info->d_cursor);
         OPS_CUDA(h, cudaGetLastError());
     }
-    int c_nnz = 0;
-    if (M > 0) OPS_CUDA(h, cudaMemcpyAsync(&c_nnz, c_rpt + M, sizeof(int), cudaMemcpyDeviceToHost, st));
-    OPS_CUDA(h, cudaMemcpyAsync(&pl.long_b_count, &h->info->d_cursor, sizeof(int), cudaMemcpyDeviceToHost, st));
-    long long products = 0;
-    OPS_CUDA(h, cudaMemcpyAsync(&products, pl.pos_base + na - (nnz_a > 0 ? 0 : 1), sizeof(long long),
+    // one round trip for the three sizes (through pinned memory: a copy to pageable memory
+    // waits for the stream)
+    struct Sizes {
+        long long products;
+        int long_b_count, c_nnz;
+    };
+    static_assert(sizeof(Sizes) <= sizeof(DevInfo), "the handle's pinned record holds the sizes");
+    Sizes *sizes = reinterpret_cast<Sizes *>(h->h_info);
+    if (M > 0) OPS_CUDA(h, cudaMemcpyAsync(&sizes->c_nnz, c_rpt + M, sizeof(int), cudaMemcpyDeviceToHost, st));
+    OPS_CUDA(h, cudaMemcpyAsync(&sizes->long_b_count, &h->info->d_cursor, sizeof(int), cudaMemcpyDeviceToHost, st));
+    OPS_CUDA(h, cudaMemcpyAsync(&sizes->products, pl.pos_base + na - (nnz_a > 0 ? 0 : 1), sizeof(long long),
                                 cudaMemcpyDeviceToHost, st));
     OPS_CUDA(h, cudaStreamSynchronize(st));
-    if (nnz_a == 0) products = 0;
+    const int c_nnz = M > 0 ? sizes->c_nnz : 0;
+    const long long products = nnz_a > 0 ? sizes->products : 0;
+    pl.long_b_count = sizes->long_b_count;
     pl.products = products;
     // blocks of rows for dB's gathers
     pl.blocks = (int)std::min<long long>(std::min<long long>(((long long)c_nnz + kGradBlock - 1) / kGradBlock, kGradBlocksMax),
@@ -565,7 +573,11 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
         OPS_CUDA(h, cudaGetLastError());
     }
     OPS_CUDA(h, cudaFreeAsync(tp, st));
-    OPS_CUDA(h, cudaStreamSynchronize(st));  // the next call may use the plan from another stream
+    // a call on another stream waits for the plan first (settle_plan)
+    if (!pl.ready) OPS_CUDA(h, cudaEventCreateWithFlags(&pl.ready, cudaEventDisableTiming));
+    OPS_CUDA(h, cudaEventRecord(pl.ready, st));
+    OPS_CUDA(h, cudaStreamGetId(st, &pl.stream));
+    pl.settled = false;
     pl.M = M;
     pl.K = K;
     pl.N = N;
@@ -578,6 +590,29 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
     pl.c_rpt = c_rpt;
     pl.c_col = c_col;
     pl.valid = true;
+    return OPS_OK;
+}
+
+// Waits, once per plan, until the plan is complete where st does not run behind its kernels:
+// another stream than theirs, or a captured one, whose graph may run on any.  The wait is
+// allowed while st is captured, as the event lies outside the capture.
+int settle_plan(ops_handle_s *h, cudaStream_t st)
+{
+    BackwardPlan &pl = h->bwd;
+    if (pl.settled) return OPS_OK;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    OPS_CUDA(h, cudaStreamIsCapturing(st, &capture));
+    if (capture == cudaStreamCaptureStatusNone) {
+        unsigned long long id = 0;
+        OPS_CUDA(h, cudaStreamGetId(st, &id));
+        if (id == pl.stream) return OPS_OK;
+    }
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OPS_CUDA(h, cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t waited = cudaEventSynchronize(pl.ready);
+    OPS_CUDA(h, cudaThreadExchangeStreamCaptureMode(&mode));
+    OPS_CUDA(h, waited);
+    pl.settled = true;
     return OPS_OK;
 }
 
@@ -680,6 +715,7 @@ extern "C" int ops_spgemm_backward(ops_handle_t h, int dtype, int32_t rows_a, in
             h->info = reinterpret_cast<DevInfo *>(h->ws);
         }
         OPS_CHECK(build_plan(h, rows_a, cols_a, cols_b, a_rpt, a_col, a_nnz, b_rpt, b_col, b_nnz, c_rpt, c_col, st));
+        OPS_CHECK(settle_plan(h, st));
         OPS_CUDA(h, cudaMemsetAsync(&h->info->flags, 0, sizeof(int), st));
         int s;
         if (dtype == OPS_F64)

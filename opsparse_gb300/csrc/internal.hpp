@@ -34,6 +34,9 @@ struct BackwardPlan {
     int long_b_count = 0;
     int blocks = 1;                 // blocks of A's rows dB is walked in
     int *at_blk = nullptr;          // [blocks - 1][K] where the later blocks start in A's columns
+    cudaEvent_t ready = nullptr;    // recorded behind the plan's kernels
+    unsigned long long stream = 0;  // id of the stream they run on
+    bool settled = false;           // they are known to have ended
 };
 
 struct ops_handle_s {

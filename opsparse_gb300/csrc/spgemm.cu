@@ -986,6 +986,7 @@ int ops_handle_destroy(ops_handle_t h)
     if (h->bwd.mem) cudaFree(h->bwd.mem);
     if (h->bwd.pmap) cudaFree(h->bwd.pmap);
     if (h->bwd.at_blk) cudaFree(h->bwd.at_blk);
+    if (h->bwd.ready) cudaEventDestroy(h->bwd.ready);
     for (int c = 0; c < kNumClasses; ++c) {
         if (h->side[c]) cudaStreamDestroy(h->side[c]);
         if (h->ev_join[c]) cudaEventDestroy(h->ev_join[c]);

@@ -71,6 +71,37 @@ def test_two_streams_at_once(cuda, blocks):
     p.h.close()
 
 
+@pytest.mark.parametrize("how", ["stream", "graph"])
+def test_new_plan_on_another_stream(cuda, how):
+    """A plan that was just built, used at once on another stream, or by a graph that was captured
+    on its own stream and runs on another."""
+    p = Product(cuda, 6000, 800, 4000, 30, 90)
+    own, other = cuda.cuda.Stream(), cuda.cuda.Stream()
+    dc, outs = p.dc(), [p.outputs(), p.outputs()]
+    cuda.cuda.synchronize()
+    for _ in range(4):
+        capi.check(p.h.lib.ops_handle_set_map_budget(p.h.h, 8 << 30))  # drops the plan
+        for t in outs[1]:
+            t.fill_(np.nan)
+        cuda.cuda.synchronize()
+        p.call(dc, *outs[0], own)
+        if how == "stream":
+            p.call(dc, *outs[1], other)
+        else:
+            graph = cuda.cuda.CUDAGraph()
+            with cuda.cuda.stream(own):
+                graph.capture_begin()
+                p.call(dc, *outs[1], own)
+                graph.capture_end()
+            with cuda.cuda.stream(other):
+                graph.replay()
+        cuda.cuda.synchronize()
+        capi.check(p.h.lib.ops_spgemm_check(p.h.h, ops._stream_ptr()), p.h.h)
+        p.check(dc, *outs[1])
+        graph = None
+    p.h.close()
+
+
 def test_captured_call(cuda):
     """A built plan's call in a graph, replayed with new dC; C of more entries than one block."""
     p = Product(cuda, 5000, 6000, 5000, 36, 140)
