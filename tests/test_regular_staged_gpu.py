@@ -119,3 +119,27 @@ def test_numeric_on_a_one_pass_plan(cuda, name, dtype):
                     c_val = cuda.full((nnz,), 7.0, dtype=A.val.dtype, device="cuda")
                     h.numeric(A2, B2, c_rpt, nnz, c_col=c_col, c_val=c_val)
                     check((want[0], c_col.cpu().numpy(), c_val.cpu().numpy()), expect)
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+def test_repeated_columns_of_b_are_not_grouped(cuda, dtype):
+    """B rows that hold a column twice are outside the library's contract: the values are then
+    undefined, but C's pattern is the product's, as it is for rows of every other class."""
+    rows, offs_a, offs_b = 25000, np.arange(10), np.array([0, 1, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 13, 14, 15])
+    k = rows + 10
+    tdt = cuda.float64 if dtype == "f64" else cuda.float32
+
+    def band(n, offs):
+        return ((np.arange(n + 1) * len(offs)).astype(np.int32),
+                (np.arange(n)[:, None] + offs[None, :]).astype(np.int32).ravel(), np.ones(n * len(offs)))
+
+    A = ops.csr_to_device(*band(rows, offs_a), rows, k, dtype=tdt)
+    B = ops.csr_to_device(*band(k, offs_b), k, k + 16, dtype=tdt)
+    want = band(rows, np.arange(25))
+    for mode in (0, 1, 2):
+        with ops.Handle() as h:
+            h.set_one_pass(mode)
+            for multiply in (h.spgemm, h.spgemm_oneshot):
+                rpt, col, _ = multiply(A, B).to_host()
+                assert np.array_equal(rpt, want[0]) and np.array_equal(col, want[1])
+                assert grouped_rows(h) == 0
