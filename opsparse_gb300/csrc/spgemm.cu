@@ -372,14 +372,15 @@ int form_groups(ops_handle_s *h, DevInfo &hi, const Mat &A, const Mat &B, bool w
         h->b_link_rows = K;
     }
     const int sms = h->num_sms;
+    const bool unstage = want_stage && hi.e1_one > 0;  // else no row stages: no sizes to look at
     k_shift_links<<<grid_for(K, 32, sms * 16), 256, 0, st>>>(B.rpt, B.col, K, B.cols, h->b_link);
     k_row_links<<<grid_for(M, 32, sms * 16), 256, 0, st>>>(A.rpt, A.col, B.rpt, M, h->b_link, h->link);
     k_form_groups<<<(M + 4 * kGroupWindow - 1) / (4 * kGroupWindow), 128, 0, st>>>(
-        M, h->link, h->groups, want_stage ? h->soff : nullptr, h->info);
+        M, h->link, h->groups, unstage ? h->soff : nullptr, h->info);
     OPS_CUDA(h, cudaGetLastError());
     h->launches += 3;
     h->regular = true;
-    if (want_stage && hi.e1_one > 0) {
+    if (unstage) {
         OPS_CUDA(h, cudaMemcpyAsync(h->h_info, h->info, sizeof(DevInfo), cudaMemcpyDeviceToHost, st));
         OPS_CUDA(h, cudaStreamSynchronize(st));
         hi.staged_flop = h->h_info->staged_flop;
