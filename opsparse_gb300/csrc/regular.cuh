@@ -427,6 +427,7 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupCtas) k_group_rows(Spgemm
     const int warp = t >> 5;
     const int count = g.info->groups;
     const int levels = rank_levels(g.N, kGroupTop);
+    const int a_nnz = __ldg(g.arpt + g.M), b_nnz = __ldg(g.brpt + g.K);
     for (;;) {
         if (t == 0) s.next = atomicAdd(cursor, 1);
         __syncthreads();
@@ -444,11 +445,22 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupCtas) k_group_rows(Spgemm
             b0 = __ldg(g.brpt + j);
             bl = __ldg(g.brpt + j + 1) - b0;
         }
-        const int jp = __shfl_up_sync(kFull, j, 1);
+        const int jp = __shfl_up_sync(kFull, j, 1), lp = __shfl_up_sync(kFull, bl, 1);
         const bool head = lane < len_a && (lane == 0 || jp != j - 1);
         const unsigned heads = __ballot_sync(kFull, head);
         const int pencils = __popc(heads);
         const int longest = (int)__reduce_max_sync(kFull, (unsigned)bl);
+        // what the reads and the shared memory below rest on; the groups were formed so
+        const bool same = (unsigned)(len_a - 1) < (unsigned)kGroupAMax &&
+                          (unsigned)longest <= kGroupStage / kGroupLanes &&
+                          (len_a + pencils * (kGroupLanes - 1)) * (longest | 1) + 8 * pencils <= kGroupStage &&
+                          gr.y * len_a <= a_nnz - a0 && gr.y * bl <= b_nnz - b0 &&
+                          (lane >= len_a || head || lp == bl);
+        if (!__all_sync(kFull, same)) {  // not the matrices that were classified (on every warp alike)
+            if (t == 0) atomicOr(&g.info->flags, kErrCountMismatch);
+            __syncthreads();  // s.next is read
+            continue;
+        }
         // B rows of one odd length: a pencil's rows lie in b as they lie in B, copied 16 bytes
         // at a time; else every B row gets a row of an odd pitch
         const bool packed = (longest & 1) && __all_sync(kFull, lane >= len_a || bl == longest);
@@ -572,7 +584,7 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupCtas) k_group_rows(Spgemm
             }
         }
         __syncthreads();
-        rank_prefix<NT>(mask, s.start, total, t, warp, lane, s.wsum);
+        const int listed = rank_prefix<NT>(mask, s.start, total, t, warp, lane, s.wsum);
 #pragma unroll
         for (int k = 0; k < PER; ++k) {
             if (t + k * NT < products) {
@@ -592,7 +604,7 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupCtas) k_group_rows(Spgemm
             }
             s.part[t] = lo;
         }
-        const bool fits = __ldg(g.c_rpt + gr.x + gr.y) - off == gr.y * total;
+        const bool fits = __ldg(g.c_rpt + gr.x + gr.y) - off == gr.y * total && listed == s.e_start[len_a];
         if (t == 0 && !fits) atomicOr(&g.info->flags, kErrCountMismatch);
         int n = 0;
         for (int r0 = 0; r0 < gr.y; r0 += n) {

@@ -143,3 +143,39 @@ def test_repeated_columns_of_b_are_not_grouped(cuda, dtype):
                 rpt, col, _ = multiply(A, B).to_host()
                 assert np.array_equal(rpt, want[0]) and np.array_equal(col, want[1])
                 assert grouped_rows(h) == 0
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("which", ["a", "b"])
+def test_changed_matrices_are_refused(cuda, dtype, which):
+    """Row pointers that changed behind the plan's back (still those of a CSR matrix): the group
+    that they belong to raises the mismatch that the other classes' rows raise, and the same call
+    on the matrices of the plan is right again."""
+    offs_a, offs_b = np.arange(25), np.arange(0, 40, 2)
+    rows = 25000  # 24 windows of 1,024 rows and 424 rows: all of them in groups
+    k = rows + 25
+    rng = np.random.default_rng(2)
+    npdt = np.float64 if dtype == "f64" else np.float32
+
+    def band(n, offs):
+        return ((np.arange(n + 1) * len(offs)).astype(np.int32),
+                (np.arange(n)[:, None] + offs[None, :]).astype(np.int32).ravel(),
+                rng.standard_normal(n * len(offs)).astype(npdt))
+
+    a, b, ncols = band(rows, offs_a), band(k, offs_b), k + 40
+    tdt = cuda.float64 if dtype == "f64" else cuda.float32
+    A, B = ops.csr_to_device(*a, rows, k, dtype=tdt), ops.csr_to_device(*b, k, ncols, dtype=tdt)
+    want = oracle.spgemm(*a, *b, ncols, dtype=npdt)
+    with ops.Handle() as h:
+        c_rpt, nnz = h.symbolic(A, B)
+        changed = (A if which == "a" else B).rpt
+        before = changed[1:2].clone()
+        # row 0 takes entries of row 1: 40 entries of A, more than a group's rows may have; 35 of B
+        changed[1] = 40 if which == "a" else 35
+        with pytest.raises(ops.OpsError) as e:
+            h.numeric(A, B, c_rpt, nnz)
+        assert e.value.status == ops.capi.OPS_COUNT_MISMATCH
+        changed[1:2] = before
+        c_col, c_val = h.numeric(A, B, c_rpt, nnz)
+        check((c_rpt.cpu().numpy(), c_col.cpu().numpy(), c_val.cpu().numpy()), want)
+        assert grouped_rows(h) == rows
