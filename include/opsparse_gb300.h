@@ -76,7 +76,8 @@ typedef struct {
 int ops_handle_create(ops_handle_t *handle);
 int ops_handle_destroy(ops_handle_t handle);
 /* Event timing: 0 off, 1 per phase, 2 per phase and per class kernel (events recorded on
- * each class's own stream around its kernel). */
+ * each class's own stream around its kernel; small problems, which otherwise run one kernel
+ * for all classes, then run the classes' kernels: the breakdown is of those). */
 int ops_handle_set_timing(ops_handle_t handle, int enable);
 int ops_handle_get_timings(ops_handle_t handle, ops_timings *out);
 /* Upper bound in bytes for the dense-row scratch (default 4 GiB). */
@@ -91,9 +92,10 @@ int ops_handle_set_output_malloc(ops_handle_t handle, int use_cuda_malloc);
  * area held by the handle and copied into C after the row_ptr scan, instead of reading A
  * and B again in a second pass.  Left to two passes: the R8 rows (counted while they are
  * classified, computed straight into C), the E1 rows whose products fall within 32768
- * consecutive columns (banded and stencil rows, which fold many products per output), and
- * the D rows when their whole-GPU sort would exceed the dense-row budget.  The staging area grows only and holds the eligible
- * products (column and value each), at most the staging budget (2 GiB unless
+ * consecutive columns (banded and stencil rows, which fold many products per output) or that
+ * are computed in groups of one pattern (structured grids), and the D rows when their
+ * whole-GPU sort would exceed the dense-row budget.  The staging area grows only and holds the
+ * eligible products (column and value each), at most the staging budget (2 GiB unless
  * ops_handle_set_stage_budget says otherwise); beyond that, or if it cannot be allocated,
  * the call runs two passes.  mode 2: the same at any size.  mode 0: always two
  * passes.  Results are identical in every mode.  ops_spgemm_symbolic and

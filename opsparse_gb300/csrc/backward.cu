@@ -40,9 +40,10 @@ namespace {
 
 constexpr int kGradBatch = 8;      // chain steps whose operands are loaded together
 constexpr int kGradShortMax = 64;  // chains longer than this are folded by a warp
-// dB walks A's rows in blocks of at most kGradBlock entries of C (112 MB in FP64, within
-// L2), where the columns of A are long enough for a block to hold kGradBlockMean of their
-// entries on average.  Graph of 200,000 nodes times its transpose (40 million entries): the
+// dB walks A's rows in blocks of about kGradBlock entries of C (112 MB in FP64, within L2; in
+// FP32 half of it), but in no more than kGradBlocksMax and only as many as leave a block
+// kGradBlockMean entries of A's columns on average: of a C of more than 8 x 14.7 million
+// entries, or of short columns, the blocks are larger and reach beyond L2.  Graph of 200,000 nodes times its transpose (40 million entries): the
 // gradient kernel 557 us in one block, 470 in five, 391 in three, 375 in three with half the
 // operands loaded ahead (a block's part of a column is short), the step 3.21 -> 3.00 ms;
 // uniform 100,000 x 60,000 x 100,000 FP32, the step 1.18 -> 0.80 ms with what a thread per

@@ -31,7 +31,7 @@
 // three dependent loads (A's column, B's row extent, B's column).  Measured on a GB300
 // against the register, CTA and radix sorts that it replaced: rows of 129-512 products of a
 // batch 331 -> 255 us, 513-1,024 141 -> 110, rows of 1,025-4,096 products 82 -> 36 us
-// (web graph of 300,000 rows, FP32), 4,097-13,312 55 -> 73 (only 40 rows: one chain each).
+// (web graph of 300,000 rows, FP32), 4,097-13,312 55 -> 43 (only 40 rows: one chain each).
 #pragma once
 
 #include <climits>

@@ -24,14 +24,17 @@
 //
 // What bounds it: FP64 issue (a warp's FMA occupies the SM for about 20 cycles; a 78-row
 // run of the 27-point stencil takes 2.5 FMAs per product, 0.80 ms for an 80^3 grid); FP32
-// instruction issue (80% of the slots; the compensated sum and three shared loads a
-// product), so a lane takes two rows there and the compensated sums of both in packed
-// instructions: 61x47x53 grid, the numeric phase 331 us against 283.  What is done once a
-// chunk counts as much: with every warp at every pencil of the staging and a search per warp
-// for its share the kernel took 262 million warp instructions and 268 us, without 199
-// million and 216 (a row per lane).  The warp hash, which probes and updates shared memory for every product,
-// took 1.91 ms (FP32, 61x47x53 grid: 548 us), the window count of every row
-// 0.58 ms against 0.11 for links, groups and counts.
+// instruction issue (the compensated sum and three shared loads a product), so a lane takes
+// two rows there and the compensated sums of both in packed instructions: 61x47x53 grid, the
+// kernel 216 -> 175 us, 199 -> 133 million warp instructions, 81% -> 66% of the issue slots
+// (barriers and the fixed latency of the packed instructions first), the numeric phase 331 ->
+// 283 us.  What is done once a chunk counts as much: with every warp at every pencil of the
+// staging and a search per warp for its share a row per lane took 262 million warp
+// instructions and 268 us.  The warp hash, which probes and updates shared memory for every
+// product, took 1.91 ms (FP32, 61x47x53 grid: 548 us), the window count of every row 0.58 ms
+// against 0.11 for links, groups and counts.  Rows that one-pass calls would stage (products
+// over 32,768 columns or more) gain as much: 25x100x100 grid, FP64, one call 0.85 ms, two
+// phases 0.72 ms, against 4.7 and 1.7 ms by sort and hash kernels.
 #pragma once
 
 #include <type_traits>
