@@ -93,14 +93,22 @@ __global__ void k_iota(int *out, long long n)
         out[p] = (int)p;
 }
 
-// arow[p] = row of entry p < nnz; one warp per row.
-__global__ void k_expand_rows(const int *__restrict__ arpt, int M, long long nnz, int *__restrict__ arow)
+// arow[p] = row of A's entry p < nnz_a, brow[q] = row of B's entry q < nnz_b; one warp per row.
+// *count = 0.
+__global__ void k_expand_rows(const int *__restrict__ arpt, int M, long long nnz_a, int *__restrict__ arow,
+                              const int *__restrict__ brpt, int K, long long nnz_b, int *__restrict__ brow, int *count)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *count = 0;
     const long long w0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long i = w0; i < M; i += nw) {
-        const int a0 = __ldg(arpt + i), a1 = __ldg(arpt + i + 1);
-        for (int p = a0 + lane_id(); p < a1 && p < nnz; p += 32) arow[p] = (int)i;
+    for (long long w = w0; w < (long long)M + K; w += nw) {
+        const bool of_a = w < M;
+        const int i = (int)(of_a ? w : w - M);
+        const int *rpt = of_a ? arpt : brpt;
+        int *row = of_a ? arow : brow;
+        const long long nnz = of_a ? nnz_a : nnz_b;
+        const int p0 = __ldg(rpt + i), p1 = __ldg(rpt + i + 1);
+        for (int p = p0 + lane_id(); p < p1 && p < nnz; p += 32) row[p] = i;
     }
 }
 
@@ -501,18 +509,15 @@ int build_plan(ops_handle_s *h, int M, int K, int N, const int *a_rpt, const int
         OPS_CUDA(h, cudaGetLastError());
     }
     OPS_CUDA(h, cub::DeviceScan::ExclusiveSum(scan_scratch, scan_tmp, blen, pl.pos_base, (int)na + 1, st));
-    if (M > 0) {
-        k_expand_rows<<<grid_of(M, 8, sms * 8), 256, 0, st>>>(a_rpt, M, nnz_a, pl.arow);
-        OPS_CUDA(h, cudaGetLastError());
-    }
+    k_expand_rows<<<grid_of((long long)M + K, 8, sms * 8), 256, 0, st>>>(a_rpt, M, nnz_a, pl.arow, b_rpt, K, nnz_b,
+                                                                         pl.brow, &h->info->d_cursor);
+    OPS_CUDA(h, cudaGetLastError());
     if (nnz_a > 0)
         OPS_CUDA(h, cub::DeviceRadixSort::SortPairs(sort_scratch, sort_tmp, a_col, sorted_cols, iota, pl.at_ent,
                                                     (int)nnz_a, 0, std::max(1, ceil_log2(std::max(K, 2))), st));
     k_col_starts<<<grid_of(nnz_a + 1, 256, sms * 16), 256, 0, st>>>(sorted_cols, nnz_a, K, pl.at_ptr);
     OPS_CUDA(h, cudaGetLastError());
-    OPS_CUDA(h, cudaMemsetAsync(&h->info->d_cursor, 0, sizeof(int), st));
     if (nnz_b > 0) {
-        k_expand_rows<<<grid_of(K, 8, sms * 8), 256, 0, st>>>(b_rpt, K, nnz_b, pl.brow);
         k_list_long_b<<<grid_of(nnz_b, 256, sms * 16), 256, 0, st>>>(nnz_b, pl.brow, b_rpt, pl.at_ptr, pl.long_b,
                                                                      &h->info->d_cursor);
         OPS_CUDA(h, cudaGetLastError());

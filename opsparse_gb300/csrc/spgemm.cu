@@ -683,7 +683,7 @@ int count_status(ops_handle_s *h, const DevInfo &d)
 // against 133, where the scan by one CTA also ends.  Rows of 96, 140 and 224 products each:
 // 8,000 of them 101, 105 and 114 us against 112, 135 and 142; 32,000 150, 181 and 204 against
 // 158, 208 and 230.  The mean decides for want of the largest row, which must not pass 256
-// products: above it the two launches were for nothing (500 rows 172 us against 168).
+// products: above it the two launches were for nothing (500 rows 176 us against 168).
 constexpr int kSmallRows = 16384;
 constexpr double kSmallMeanProducts = 96;
 
