@@ -87,9 +87,11 @@ def grouped_rows(h):
 def test_grouped_rows_are_not_staged(cuda, name, dtype):
     a, b, A, B, want = on_device(cuda, name, dtype)
     other = cuda.cuda.Stream()
-    for mode in (1, 2, 0):
+    for mode, budget in ((1, None), (2, None), (2, 0), (0, None)):
         with ops.Handle() as h:
             h.set_one_pass(mode)
+            if budget is not None:  # what is left to stage does not fit: two passes after all
+                h.set_stage_budget(budget)
             for stream in (None, other):
                 check(h.spgemm_oneshot(A, B, stream=stream).to_host(), want)
                 assert grouped_rows(h) > A.rows // 4
