@@ -680,7 +680,7 @@ int count_status(ops_handle_s *h, const DevInfo &d)
 // Whether a problem is launched as a small one: few rows, short ones on average.  One kernel
 // against the classes' (FP64, two phases, a 5-point grid of 128 columns): 4,096 rows 81 us
 // against 106, 8,192 96 against 107, 16,384 106 against 115, 24,576 126 against 133, 32,640 131
-// against 133, where the scan by one CTA also ends.  Rows of 96, 140 and 224 products each:
+// against 133, all of them scanned by one CTA, which stops paying at 16,384.  Rows of 96, 140 and 224 products each:
 // 8,000 of them 101, 105 and 114 us against 112, 135 and 142; 32,000 150, 181 and 204 against
 // 158, 208 and 230.  The mean decides for want of the largest row, which must not pass 256
 // products: above it the two launches were for nothing (500 rows 176 us against 168).
